@@ -1,6 +1,7 @@
 // Matvec kernels for the MFS operator K (nf collocation rows x n sources).
 //
-//  * point kernel, evaluated in registers:
+//  * point kernel, evaluated in registers (FP32 here; the FP64 products are
+//    matvec64.cuh's):
 //      K(i,j) = coef ((x_i - y_j).n_i) / |x_i - y_j|^3   (src/kernels.h:24-40)
 //    rows   : W[i, r] = sum_j K(i,j) V[j, r]   (one row per thread, sources
 //             staged through shared memory in tiles, R columns per chunk)
@@ -20,18 +21,6 @@
 
 namespace mbc {
 
-// Reciprocal square root to FP64 accuracy: FP32 hardware estimate refined by
-// two Newton-Raphson steps y <- y (3 - a y^2) / 2, written as
-// e = 1 - a y^2 (one FMA), y <- y + (y/2) e.  Valid for a in FP32 range.
-__device__ __forceinline__ double rsqrt_nr(double a)
-{
-  double y = (double)rsqrtf((float)a);
-  double e = fma(-a * y, y, 1.0);
-  y = fma(0.5 * y, e, y);
-  e = fma(-a * y, y, 1.0);
-  return fma(0.5 * y, e, y);
-}
-
 template <typename T>
 struct PointKernel;
 
@@ -47,34 +36,49 @@ struct PointKernel<float> {
   }
 };
 
+// FP64 kernel value rn a^(-3/2), a = |x - y|^2, in 16 FP64 instructions: the
+// FP32 hardware estimate y0 of a^(-1/2) has e = 1 - a y0^2 with |e| < 1e-6
+// (its own error and the rounding of a to FP32), and
+// a^(-3/2) = y0^3 (1 - e)^(-3/2) = y0^3 (1 + 3/2 e + 15/8 e^2 + O(e^3)), the
+// dropped term below 3e-18.  Two Newton-Raphson steps on a^(-1/2) and its
+// cube take 20.  Valid for a in FP32 range; a = 0 gives NaN.
 template <>
 struct PointKernel<double> {
+  __device__ __forceinline__ static double eval(const double3 &x, const double3 &nx, const double3 &y)
+  {
+    const double dx = x.x - y.x, dy = x.y - y.y, dz = x.z - y.z;
+    const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+    const double rn = fma(dz, nx.z, fma(dy, nx.y, dx * nx.x));
+    const double y0 = (double)rsqrtf((float)r2);
+    const double y2 = y0 * y0;
+    const double e = fma(-r2, y2, 1.0);
+    const double s = rn * y0 * y2;
+    return fma(s, e * fma(e, 1.875, 1.5), s);
+  }
   __device__ __forceinline__ static double eval(const float4 &x, const float4 &nx, const float4 &y)
   {
-    const double dx = (double)x.x - (double)y.x, dy = (double)x.y - (double)y.y,
-                 dz = (double)x.z - (double)y.z;
-    const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-    const double ir = rsqrt_nr(r2);
-    const double rn = fma(dz, (double)nx.z, fma(dy, (double)nx.y, dx * (double)nx.x));
-    return rn * (ir * ir * ir);
+    return eval(make_double3(x.x, x.y, x.z), make_double3(nx.x, nx.y, nx.z), make_double3(y.x, y.y, y.z));
   }
 };
 
 // Single-layer potential kernel 1/|x - y| in FP64 (the normal is unused):
-// the potential of the solved strengths, utils/torch_utils.py:254-276.
+// the potential of the solved strengths, utils/torch_utils.py:254-276.  The
+// same expansion: a^(-1/2) = y0 (1 + e/2 + 3/8 e^2 + O(e^3)).
 struct SingleLayer64 {
-  __device__ __forceinline__ static double eval(const float4 &x, const float4 &, const float4 &y)
+  __device__ __forceinline__ static double eval(const double3 &x, const double3 &, const double3 &y)
   {
-    const double dx = (double)x.x - (double)y.x, dy = (double)x.y - (double)y.y,
-                 dz = (double)x.z - (double)y.z;
-    return rsqrt_nr(fma(dz, dz, fma(dy, dy, dx * dx)));
+    const double dx = x.x - y.x, dy = x.y - y.y, dz = x.z - y.z;
+    const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+    const double y0 = (double)rsqrtf((float)r2);
+    const double e = fma(-r2, y0 * y0, 1.0);
+    return fma(y0, e * fma(e, 0.375, 0.5), y0);
   }
 };
 
 // Rows direction.  Block = TI threads, one row each; grid.x over rows,
 // grid.y over RC-column chunks.  `done` (may be NULL) lets an iteration that
 // has nothing left to do exit at once.
-template <typename T, int RC, int TI, int TJ, class Ker = PointKernel<T>>
+template <typename T, int RC, int TI, int TJ>
 __global__ void __launch_bounds__(TI) pk_rows_kernel(
     const float4 *__restrict__ xr, const float4 *__restrict__ nr, int nf,
     const float4 *__restrict__ ys, int n, const T *__restrict__ v, int ldv,
@@ -106,13 +110,13 @@ __global__ void __launch_bounds__(TI) pk_rows_kernel(
     if (jm == TJ) {
 #pragma unroll 2
       for (int jj = 0; jj < TJ; ++jj) {
-        const T k = Ker::eval(xi, ni, sy[jj]);
+        const T k = PointKernel<T>::eval(xi, ni, sy[jj]);
 #pragma unroll
         for (int r = 0; r < RC; ++r) acc[r] = fma(k, sv[jj * RC + r], acc[r]);
       }
     } else {
       for (int jj = 0; jj < jm; ++jj) {
-        const T k = Ker::eval(xi, ni, sy[jj]);
+        const T k = PointKernel<T>::eval(xi, ni, sy[jj]);
 #pragma unroll
         for (int r = 0; r < RC; ++r) acc[r] = fma(k, sv[jj * RC + r], acc[r]);
       }

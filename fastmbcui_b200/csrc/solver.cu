@@ -18,6 +18,7 @@
 #include "factor_tc.cuh"
 #include "forces.cuh"
 #include "matvec.cuh"
+#include "matvec64.h"
 #include "matvec_mesh.cuh"
 #include "matvec_tc.cuh"
 #include "cuda_util.h"
@@ -101,9 +102,11 @@ template <typename T, int RC, int TI>
 void rows_launch(const Solver &S, int R, const T *v, T *w, const int32_t *done, cudaStream_t st)
 {
   if (S.op.kind == MBC_OP_POINT_KERNEL) {
-    dim3 grid(cdiv(S.nf, TI), cdiv(R, RC));
-    pk_rows_kernel<T, RC, TI, TJ_ROWS><<<grid, TI, 0, st>>>(S.x4(), S.n4(), S.nf, S.y4(), S.n, v, R,
-                                                            (T)S.op.coef, w, R, R, done);
+    if constexpr (sizeof(T) == 4) {  // FP64: matvec64.cu
+      dim3 grid(cdiv(S.nf, TI), cdiv(R, RC));
+      pk_rows_kernel<T, RC, TI, TJ_ROWS><<<grid, TI, 0, st>>>(S.x4(), S.n4(), S.nf, S.y4(), S.n, v, R,
+                                                              (T)S.op.coef, w, R, R, done);
+    }
   } else if (S.op.kind == MBC_OP_MESH) {
     dim3 grid(cdiv(S.nf, TI), cdiv(R, RC));
     mesh_rows_kernel<T, RC, TI, TJ_ROWS><<<grid, TI, 0, st>>>(S.x4(), S.n4(), S.z4(), S.nf, S.y4(), S.n, v, R,
@@ -121,8 +124,9 @@ int cols_launch(const Solver &S, int R, const T *w, T *t, const T *pdot, double 
 {
   dim3 grid(cdiv(S.n, TI), cdiv(R, RC));
   if (S.op.kind == MBC_OP_POINT_KERNEL) {
-    pk_cols_kernel<T, RC, TI, TJ_COLS><<<grid, TI, 0, st>>>(S.x4(), S.n4(), S.nf, S.y4(), S.n, w, R,
-                                                            (T)S.op.coef, t, R, R, pdot, part, done);
+    if constexpr (sizeof(T) == 4)
+      pk_cols_kernel<T, RC, TI, TJ_COLS><<<grid, TI, 0, st>>>(S.x4(), S.n4(), S.nf, S.y4(), S.n, w, R,
+                                                              (T)S.op.coef, t, R, R, pdot, part, done);
   } else if (S.op.kind == MBC_OP_MESH) {
     mesh_cols_kernel<T, RC, TI, TJ_COLS><<<grid, TI, 0, st>>>(S.x4(), S.n4(), S.z4(), S.nf, S.y4(), S.n, w, R,
                                                               (T)S.op.coef, t, R, R, pdot, part, done);
@@ -202,6 +206,7 @@ void launch_rows(const Solver &S, int R, const T *v, T *w, const int32_t *done, 
       oz_launch_rows(S, R, v, w, done, st);
       return;
     }
+    if (S.op.kind == MBC_OP_POINT_KERNEL) return p64_launch_rows(S, R, v, w, done, st);
   }
   ++S.launches;
   const Shape sh = pick_shape<T>(S.op.kind != MBC_OP_DENSE ? S.nf : 1 << 30, R);
@@ -226,6 +231,7 @@ int launch_cols(const Solver &S, int R, const T *w, T *t, const T *pdot, double 
     }
   } else {
     if (use_oz(S)) return oz_launch_cols(S, R, w, t, pdot, part, done, st);
+    if (S.op.kind == MBC_OP_POINT_KERNEL) return p64_launch_cols(S, R, w, t, pdot, part, done, st);
   }
   ++S.launches;
   const Shape sh = pick_shape<T>(S.n, R);
@@ -240,8 +246,8 @@ int launch_cols(const Solver &S, int R, const T *w, T *t, const T *pdot, double 
 }
 
 // upper bound on the blocks of any columns-direction launch (the per-block
-// curvature partials): SIMT tiles of 64 sources or more, tensor cores 128
-int cols_blocks(const Solver &S) { return (int)cdiv(S.n, 64); }
+// curvature partials): FP64 tiles of 16 sources or more, SIMT 64, tensor cores 128
+int cols_blocks(const Solver &S) { return p64_part_rows(S.n); }
 
 template void launch_rows<float>(const Solver &, int, const float *, float *, const int32_t *, cudaStream_t);
 template void launch_rows<double>(const Solver &, int, const double *, double *, const int32_t *, cudaStream_t);
@@ -615,6 +621,7 @@ static mbc_status pcg_buffers_in(Solver &S, int R, PcgWork<T> &w, DevMem &m, Dev
   w.sc.stall = ii + 2 * R + 4;
   w.sc.drop2 = 0.0;
   w.sc.stall_check = 1;
+  if (sizeof(T) == 8) p64_reserve(S, R);  // without the buffer the products run unsplit
   return MBC_OK;
 }
 
@@ -2073,13 +2080,7 @@ extern "C" mbc_status mbc_added_mass(mbc_solver *s, int32_t R, const void *X, in
   MBC_CK(cudaMemcpyAsync(dcen.ptr, centers, sizeof(double) * 3 * n_bodies, cudaMemcpyHostToDevice, st));
   // phi = SL X in FP64 (strengths gathered into the plan order of the sources)
   mbc::permute_in<double>(S, R, X, x_dtype, (double *)xp.ptr, st);
-  {
-    constexpr int RC = 16, TI = 64;
-    dim3 grid(mbc::cdiv(S.nf, TI), mbc::cdiv(R, RC));
-    mbc::pk_rows_kernel<double, RC, TI, mbc::TJ_ROWS, mbc::SingleLayer64><<<grid, TI, 0, st>>>(
-        S.x4(), S.n4(), S.nf, S.y4(), S.n, (const double *)xp.ptr, R, 1.0 / (4.0 * 3.14159265358979323846),
-        (double *)phi.ptr, R, R, nullptr);
-  }
+  mbc::p64_launch_potential(S, R, (const double *)xp.ptr, (double *)phi.ptr, st);
   mbc::added_mass_kernel<<<dim3(n_bodies, mbc::cdiv(R, 32)), 256, 0, st>>>(
       S.x4(), S.n4(), w, (const int32_t *)dptr.ptr, (const double *)dcen.ptr, (const double *)phi.ptr, R,
       rho_fluid, (double *)dmf.ptr);
