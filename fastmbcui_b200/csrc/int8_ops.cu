@@ -161,7 +161,7 @@ mbc_status mbc::Solver::ensure_oz(cudaStream_t st, int R)
   if (!oz_ready) {
     const size_t a0 = oz::adig_bytes(nf, n), a1 = oz::adig_bytes(n, nf);
     size_t free_b = 0, total_b = 0;
-    MBC_CK(cudaMemGetInfo(&free_b, &total_b));
+    MBC_CK(device_free_bytes(&free_b, &total_b));
     MBC_TRY(m_oz_aexp[0].reserve(sizeof(int32_t) * oz::aexp_count(nf, n)));
     MBC_TRY(m_oz_aexp[1].reserve(sizeof(int32_t) * oz::aexp_count(n, nf)));
     const size_t sm0 = sizeof(float4) * oz::kChunk, sm1 = 2 * sizeof(float4) * oz::kChunk;
@@ -181,7 +181,7 @@ mbc_status mbc::Solver::ensure_oz(cudaStream_t st, int R)
       if (m_oz_a[0].reserve(a0) != MBC_OK || m_oz_a[1].reserve(a1) != MBC_OK) {
         m_oz_a[0].release();
         m_oz_a[1].release();
-        MBC_CK(cudaMemGetInfo(&free_b, &total_b));
+        MBC_CK(device_free_bytes(&free_b, &total_b));
         oz_slab = true;
       }
     }
@@ -320,7 +320,8 @@ extern "C" mbc_status mbc_solver_set_fp64_matvec(mbc_solver *s, int32_t impl)
 extern "C" mbc_status mbc_solver_prepare(mbc_solver *s, mbc_stream stream)
 {
   if (!s) return fail(MBC_BAD_ARG, "NULL solver");
-  MBC_TRY(s->s.ensure_oz((cudaStream_t)stream, 1));
+  mbc::CallScope scope((cudaStream_t)stream);
+  MBC_TRY(scope.end(s->s.ensure_oz((cudaStream_t)stream, 1)));
   MBC_CK(cudaStreamSynchronize((cudaStream_t)stream));
   return MBC_OK;
 }

@@ -44,8 +44,20 @@ mbc_status build_supernodes(Plan &p, int n_threads);
 // (mbc_spatial_order).
 mbc_status spatial_order(int32_t n, const float *pts, int32_t stride, int32_t *order);
 
+// Plans and solvers alive: the last one to go empties the device memory pools
+// (devpool.h).
+void pool_retain();
+void pool_drop();
+struct PoolUser {
+  PoolUser() { pool_retain(); }
+  ~PoolUser() { pool_drop(); }
+  PoolUser(const PoolUser &) = delete;
+  PoolUser &operator=(const PoolUser &) = delete;
+};
+
 }  // namespace mbc
 
 struct mbc_plan {
+  mbc::PoolUser user;
   mbc::Plan p;
 };

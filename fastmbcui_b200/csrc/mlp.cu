@@ -174,8 +174,9 @@ struct mbc_mlp {
   std::vector<int> dims;          // n_in, hidden..., n_out
   std::vector<int64_t> woff, boff;  // offsets of W_l (dims[l+1] x dims[l]) and b_l in the parameter vector
   int64_t n_params = 0;
-  DevMem w, g, m, v, wb;          // FP32 master, gradients, Adam moments; BF16 weights
-  DevMem acts, grads, part, loss; // activations per layer (B x dims[l]), pre-activation gradients
+  // (not pooled: a forward pass returns with its kernels in flight)
+  DevMem w{false}, g{false}, m{false}, v{false}, wb{false};  // FP32 master, gradients, Adam moments; BF16 weights
+  DevMem acts{false}, grads{false}, part{false}, loss{false}; // activations per layer (B x dims[l]), pre-activation gradients
   int64_t steps = 0;
   int cap_batch = 0;
   int layers() const { return (int)dims.size() - 1; }

@@ -29,28 +29,6 @@
 
 namespace mbc {
 
-DevMem::~DevMem() { release(); }
-void DevMem::release()
-{
-  if (ptr) cudaFree(ptr);
-  ptr = nullptr;
-  bytes = 0;
-}
-mbc_status DevMem::reserve(size_t b)
-{
-  if (b <= bytes && ptr) return MBC_OK;
-  release();
-  if (b == 0) b = 16;
-  cudaError_t e = cudaMalloc(&ptr, b);
-  if (e != cudaSuccess) {
-    ptr = nullptr;
-    cudaGetLastError();
-    return fail(MBC_NO_MEMORY, std::string("cudaMalloc(") + std::to_string(b) + "): " + cudaGetErrorString(e));
-  }
-  bytes = b;
-  return MBC_OK;
-}
-
 template <typename V>
 static mbc_status upload(DevMem &m, const std::vector<V> &h, cudaStream_t st)
 {
@@ -1735,11 +1713,10 @@ extern "C" mbc_status mbc_solver_create(const mbc_plan *plan, const mbc_operator
   }
   std::unique_ptr<mbc_solver> sv(new (std::nothrow) mbc_solver());
   if (!sv) return fail(MBC_NO_MEMORY, "solver allocation failed");
-  if (cudaMallocHost((void **)&sv->s.h_flag, sizeof(int32_t) * 4) != cudaSuccess) {
-    cudaGetLastError();
-    return fail(MBC_NO_MEMORY, "pinned flag allocation failed");
-  }
-  mbc_status s = sv->s.create(plan->p, *op, precision, (cudaStream_t)stream);
+  mbc::CallScope scope((cudaStream_t)stream);
+  sv->s.h_flag = mbc::pinned_flags();
+  if (!sv->s.h_flag) return fail(MBC_NO_MEMORY, "pinned flag allocation failed");
+  mbc_status s = scope.end(sv->s.create(plan->p, *op, precision, (cudaStream_t)stream));
   if (s != MBC_OK) return s;
   *out = sv.release();
   return MBC_OK;
@@ -1747,7 +1724,7 @@ extern "C" mbc_status mbc_solver_create(const mbc_plan *plan, const mbc_operator
 
 mbc::Solver::~Solver()
 {
-  if (h_flag) cudaFreeHost(h_flag);
+  pinned_flags_release(h_flag);
   for (cudaEvent_t e : events) cudaEventDestroy(e);
 }
 
@@ -1790,7 +1767,8 @@ extern "C" mbc_status mbc_solver_destroy(mbc_solver *s)
 extern "C" mbc_status mbc_solver_factor(mbc_solver *s, mbc_stream stream)
 {
   if (!s) return fail(MBC_BAD_ARG, "NULL solver");
-  return s->s.factor((cudaStream_t)stream);
+  mbc::CallScope scope((cudaStream_t)stream);
+  return scope.end(s->s.factor((cudaStream_t)stream));
 }
 
 extern "C" void mbc_factor_default_tiles(mbc_factor_tiles *t)
@@ -1829,6 +1807,7 @@ extern "C" mbc_status mbc_solver_tune_factor(mbc_solver *s, int32_t reps, mbc_fa
   if (!s || reps < 1) return fail(MBC_BAD_ARG, "NULL solver or reps < 1");
   mbc::Solver &S = s->s;
   cudaStream_t st = (cudaStream_t)stream;
+  mbc::CallScope scope(st);
   cudaEvent_t e0, e1;
   MBC_CK(cudaEventCreate(&e0));
   MBC_CK(cudaEventCreate(&e1));
@@ -1995,7 +1974,8 @@ extern "C" mbc_status mbc_solve(mbc_solver *s, int32_t R, const void *F, int32_t
   mbc_solve_default_options(&o);
   if (opt) o = *opt;
   if (o.max_iters < 0 || !(o.tol >= 0)) return fail(MBC_BAD_ARG, "bad solve options");
-  return s->s.solve(R, F, f_dtype, X, x_dtype, X0, false, o, stats_host, iters_host, (cudaStream_t)stream);
+  mbc::CallScope scope((cudaStream_t)stream);
+  return scope.end(s->s.solve(R, F, f_dtype, X, x_dtype, X0, false, o, stats_host, iters_host, (cudaStream_t)stream));
 }
 
 extern "C" mbc_status mbc_solve_adjoint(mbc_solver *s, int32_t R, const void *B, int32_t b_dtype, void *X,
@@ -2007,7 +1987,8 @@ extern "C" mbc_status mbc_solve_adjoint(mbc_solver *s, int32_t R, const void *B,
   mbc_solve_default_options(&o);
   if (opt) o = *opt;
   if (o.max_iters < 0 || !(o.tol >= 0)) return fail(MBC_BAD_ARG, "bad solve options");
-  return s->s.solve(R, B, b_dtype, X, x_dtype, nullptr, true, o, stats_host, iters_host, (cudaStream_t)stream);
+  mbc::CallScope scope((cudaStream_t)stream);
+  return scope.end(s->s.solve(R, B, b_dtype, X, x_dtype, nullptr, true, o, stats_host, iters_host, (cudaStream_t)stream));
 }
 
 extern "C" mbc_status mbc_apply_K(mbc_solver *s, int32_t R, const void *V, void *W, mbc_stream stream)
@@ -2015,18 +1996,21 @@ extern "C" mbc_status mbc_apply_K(mbc_solver *s, int32_t R, const void *V, void 
   if (!s || R <= 0 || !V || !W) return fail(MBC_BAD_ARG, "bad arguments");
   mbc::Solver &S = s->s;
   cudaStream_t st = (cudaStream_t)stream;
-  if (S.precision == MBC_F64) {
-    MBC_TRY(S.ensure_oz(st, R));
-    MBC_TRY(S.tmp.reserve(sizeof(double) * (size_t)S.n * R));
-    mbc::permute_in<double>(S, R, V, MBC_F64, (double *)S.tmp.ptr, st);
-    mbc::launch_rows<double>(S, R, (const double *)S.tmp.ptr, (double *)W, nullptr, st);
-  } else {
-    MBC_TRY(S.tmp.reserve(sizeof(float) * (size_t)S.n * R));
-    mbc::permute_in<float>(S, R, V, MBC_F32, (float *)S.tmp.ptr, st);
-    mbc::launch_rows<float>(S, R, (const float *)S.tmp.ptr, (float *)W, nullptr, st);
-  }
-  MBC_CKL();
-  return S.check_device_error(st);
+  mbc::CallScope scope(st);
+  return scope.end([&]() -> mbc_status {
+    if (S.precision == MBC_F64) {
+      MBC_TRY(S.ensure_oz(st, R));
+      MBC_TRY(S.tmp.reserve(sizeof(double) * (size_t)S.n * R));
+      mbc::permute_in<double>(S, R, V, MBC_F64, (double *)S.tmp.ptr, st);
+      mbc::launch_rows<double>(S, R, (const double *)S.tmp.ptr, (double *)W, nullptr, st);
+    } else {
+      MBC_TRY(S.tmp.reserve(sizeof(float) * (size_t)S.n * R));
+      mbc::permute_in<float>(S, R, V, MBC_F32, (float *)S.tmp.ptr, st);
+      mbc::launch_rows<float>(S, R, (const float *)S.tmp.ptr, (float *)W, nullptr, st);
+    }
+    MBC_CKL();
+    return S.check_device_error(st);
+  }());
 }
 
 extern "C" mbc_status mbc_apply_KT(mbc_solver *s, int32_t R, const void *W, void *T, mbc_stream stream)
@@ -2034,18 +2018,21 @@ extern "C" mbc_status mbc_apply_KT(mbc_solver *s, int32_t R, const void *W, void
   if (!s || R <= 0 || !W || !T) return fail(MBC_BAD_ARG, "bad arguments");
   mbc::Solver &S = s->s;
   cudaStream_t st = (cudaStream_t)stream;
-  if (S.precision == MBC_F64) {
-    MBC_TRY(S.ensure_oz(st, R));
-    MBC_TRY(S.tmp.reserve(sizeof(double) * (size_t)S.n * R));
-    mbc::launch_cols<double>(S, R, (const double *)W, (double *)S.tmp.ptr, nullptr, nullptr, nullptr, st);
-    mbc::permute_out<double>(S, R, (const double *)S.tmp.ptr, T, MBC_F64, st);
-  } else {
-    MBC_TRY(S.tmp.reserve(sizeof(float) * (size_t)S.n * R));
-    mbc::launch_cols<float>(S, R, (const float *)W, (float *)S.tmp.ptr, nullptr, nullptr, nullptr, st);
-    mbc::permute_out<float>(S, R, (const float *)S.tmp.ptr, T, MBC_F32, st);
-  }
-  MBC_CKL();
-  return S.check_device_error(st);
+  mbc::CallScope scope(st);
+  return scope.end([&]() -> mbc_status {
+    if (S.precision == MBC_F64) {
+      MBC_TRY(S.ensure_oz(st, R));
+      MBC_TRY(S.tmp.reserve(sizeof(double) * (size_t)S.n * R));
+      mbc::launch_cols<double>(S, R, (const double *)W, (double *)S.tmp.ptr, nullptr, nullptr, nullptr, st);
+      mbc::permute_out<double>(S, R, (const double *)S.tmp.ptr, T, MBC_F64, st);
+    } else {
+      MBC_TRY(S.tmp.reserve(sizeof(float) * (size_t)S.n * R));
+      mbc::launch_cols<float>(S, R, (const float *)W, (float *)S.tmp.ptr, nullptr, nullptr, nullptr, st);
+      mbc::permute_out<float>(S, R, (const float *)S.tmp.ptr, T, MBC_F32, st);
+    }
+    MBC_CKL();
+    return S.check_device_error(st);
+  }());
 }
 
 // Added-mass tensor and fluid forces from solved strengths (see mbc.h).
@@ -2070,30 +2057,33 @@ extern "C" mbc_status mbc_added_mass(mbc_solver *s, int32_t R, const void *X, in
       return fail(MBC_BAD_ARG, "mbc_added_mass: body_ptr must ascend within [0, nf]");
   if ((R + 31) / 32 > 65535) return fail(MBC_BAD_ARG, "mbc_added_mass: R too large");
   cudaStream_t st = (cudaStream_t)stream;
-  mbc::DevMem xp, phi, dmf, dptr, dcen;
-  MBC_TRY(xp.reserve(sizeof(double) * (size_t)S.n * R));
-  MBC_TRY(phi.reserve(sizeof(double) * (size_t)S.nf * R));
-  MBC_TRY(dmf.reserve(sizeof(double) * (size_t)6 * n_bodies * R));
-  MBC_TRY(dptr.reserve(sizeof(int32_t) * (size_t)(n_bodies + 1)));
-  MBC_TRY(dcen.reserve(sizeof(double) * (size_t)3 * n_bodies));
-  MBC_CK(cudaMemcpyAsync(dptr.ptr, body_ptr, sizeof(int32_t) * (n_bodies + 1), cudaMemcpyHostToDevice, st));
-  MBC_CK(cudaMemcpyAsync(dcen.ptr, centers, sizeof(double) * 3 * n_bodies, cudaMemcpyHostToDevice, st));
-  // phi = SL X in FP64 (strengths gathered into the plan order of the sources)
-  mbc::permute_in<double>(S, R, X, x_dtype, (double *)xp.ptr, st);
-  mbc::p64_launch_potential(S, R, (const double *)xp.ptr, (double *)phi.ptr, st);
-  mbc::added_mass_kernel<<<dim3(n_bodies, mbc::cdiv(R, 32)), 256, 0, st>>>(
-      S.x4(), S.n4(), w, (const int32_t *)dptr.ptr, (const double *)dcen.ptr, (const double *)phi.ptr, R,
-      rho_fluid, (double *)dmf.ptr);
-  MBC_CKL();
-  MBC_CK(cudaMemcpyAsync(Mf, dmf.ptr, sizeof(double) * (size_t)6 * n_bodies * R, cudaMemcpyDeviceToHost, st));
-  MBC_CK(cudaStreamSynchronize(st));
-  if (accel) {
-    // reactive force of the added mass: f = -Mf a
-    for (int i = 0; i < 6 * n_bodies; ++i) {
-      double f = 0.0;
-      for (int j = 0; j < R; ++j) f += Mf[(size_t)i * R + j] * accel[j];
-      forces[i] = -f;
+  mbc::CallScope scope(st);
+  return scope.end([&]() -> mbc_status {
+    mbc::DevMem xp, phi, dmf, dptr, dcen;
+    MBC_TRY(xp.reserve(sizeof(double) * (size_t)S.n * R));
+    MBC_TRY(phi.reserve(sizeof(double) * (size_t)S.nf * R));
+    MBC_TRY(dmf.reserve(sizeof(double) * (size_t)6 * n_bodies * R));
+    MBC_TRY(dptr.reserve(sizeof(int32_t) * (size_t)(n_bodies + 1)));
+    MBC_TRY(dcen.reserve(sizeof(double) * (size_t)3 * n_bodies));
+    MBC_CK(cudaMemcpyAsync(dptr.ptr, body_ptr, sizeof(int32_t) * (n_bodies + 1), cudaMemcpyHostToDevice, st));
+    MBC_CK(cudaMemcpyAsync(dcen.ptr, centers, sizeof(double) * 3 * n_bodies, cudaMemcpyHostToDevice, st));
+    // phi = SL X in FP64 (strengths gathered into the plan order of the sources)
+    mbc::permute_in<double>(S, R, X, x_dtype, (double *)xp.ptr, st);
+    mbc::p64_launch_potential(S, R, (const double *)xp.ptr, (double *)phi.ptr, st);
+    mbc::added_mass_kernel<<<dim3(n_bodies, mbc::cdiv(R, 32)), 256, 0, st>>>(
+        S.x4(), S.n4(), w, (const int32_t *)dptr.ptr, (const double *)dcen.ptr, (const double *)phi.ptr, R,
+        rho_fluid, (double *)dmf.ptr);
+    MBC_CKL();
+    MBC_CK(cudaMemcpyAsync(Mf, dmf.ptr, sizeof(double) * (size_t)6 * n_bodies * R, cudaMemcpyDeviceToHost, st));
+    MBC_CK(cudaStreamSynchronize(st));
+    if (accel) {
+      // reactive force of the added mass: f = -Mf a
+      for (int i = 0; i < 6 * n_bodies; ++i) {
+        double f = 0.0;
+        for (int j = 0; j < R; ++j) f += Mf[(size_t)i * R + j] * accel[j];
+        forces[i] = -f;
+      }
     }
-  }
-  return S.check_device_error(st);
+    return S.check_device_error(st);
+  }());
 }

@@ -6,21 +6,10 @@
 #include <bitset>
 #include <vector>
 
+#include "devpool.h"
 #include "mbc_internal.h"
 
 namespace mbc {
-
-// Owned device allocation that only grows.
-struct DevMem {
-  void *ptr = nullptr;
-  size_t bytes = 0;
-  DevMem() = default;
-  DevMem(const DevMem &) = delete;
-  DevMem &operator=(const DevMem &) = delete;
-  ~DevMem();
-  mbc_status reserve(size_t b);
-  void release();
-};
 
 struct Solver {
   const Plan *plan = nullptr;
@@ -129,5 +118,6 @@ int launch_cols(const Solver &S, int R, const T *w, T *t, const T *pdot, double 
 
 // The C handle behind mbc_solver.
 struct mbc_solver {
+  mbc::PoolUser user;  // before s: the solver's buffers go first
   mbc::Solver s;
 };

@@ -15,7 +15,10 @@
  *   - Matrices are row-major.  A "source-space" array (n x R) is indexed by the
  *     ORIGINAL source order unless its name says otherwise.
  *   - mbc_stream is cudaStream_t; NULL is the legacy default stream.
- *   - Objects are caller-owned; the library keeps no global state.
+ *   - Objects are caller-owned.  Between solvers the library keeps idle device
+ *     memory in a pool (per device at most 8 GiB and a sixteenth of it), returned
+ *     when an allocation of its own would fail and when the last plan and
+ *     solver are destroyed; nothing else outlives the objects.
  */
 #ifndef MBC_H
 #define MBC_H
