@@ -27,7 +27,7 @@ NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr
 
 HOST_SRC = ["plan.cpp", "capi.cpp", "spatial.cpp"]
 CUDA_SRC = ["solver.cu", "context.cu", "noalloc.cu", "mlp.cu", "warmstart.cu", "mesh.cu", "int8_ops.cu", "grad.cu",
-            "matvec64.cu", "devpool.cu"]
+            "matvec64.cu", "devpool.cu", "dense.cu"]
 
 
 def _nvcc() -> str:

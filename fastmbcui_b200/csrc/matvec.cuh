@@ -7,9 +7,6 @@
 //             staged through shared memory in tiles, R columns per chunk)
 //    columns: T[j, r] = sum_i K(i,j) W[i, r]   (one source per thread, rows
 //             staged through shared memory)
-//  * dense caller matrix M (row-major float32), the mfs_torch operator input:
-//    rows   : warp per row, float4 loads of M, warp-shuffle reduction;
-//    columns: thread per column, coalesced over consecutive columns.
 //
 // Coordinates are float4 (x, y, z, 0) so every point is one 16-byte load.
 // Vectors are row-major with leading dimension `ld` (the RHS count R); a
@@ -193,104 +190,6 @@ __global__ void __launch_bounds__(TI) pk_cols_kernel(
       if (j < n && r < rc) d = (double)pdot[(size_t)j * ldt + r0 + r] * (double)acc[r];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-      if (lane == 0) sred[r][wid] = d;
-    }
-    __syncthreads();
-    if (threadIdx.x < RC && threadIdx.x < rc) {
-      double s = 0.0;
-#pragma unroll
-      for (int k = 0; k < TI / 32; ++k) s += sred[threadIdx.x][k];
-      part[(size_t)blockIdx.x * R + r0 + threadIdx.x] = s;
-    }
-  }
-}
-
-// Dense rows: W[i, r] = sum_o M[i, o] Vnew[P[o], r].  One warp per row.
-template <typename T, int RC>
-__global__ void __launch_bounds__(256) dense_rows_kernel(
-    const float *__restrict__ M, int64_t ldm, int nf, int n, const int *__restrict__ P,
-    const T *__restrict__ v, int ldv, T *__restrict__ w, int ldw, int R,
-    const int *__restrict__ done)
-{
-  if (done && *done) return;
-  const int warps = blockDim.x >> 5;
-  const int i = blockIdx.x * warps + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  const int r0 = blockIdx.y * RC;
-  const int rc = min(RC, R - r0);
-  if (i >= nf) return;
-  const float *row = M + (size_t)i * ldm;
-  T acc[RC];
-#pragma unroll
-  for (int r = 0; r < RC; ++r) acc[r] = T(0);
-  for (int o = lane; o < n; o += 32) {
-    const T m = (T)__ldg(row + o);
-    const T *vp = v + (size_t)__ldg(P + o) * ldv + r0;
-#pragma unroll
-    for (int r = 0; r < RC; ++r)
-      if (r < rc) acc[r] = fma(m, vp[r], acc[r]);
-  }
-#pragma unroll
-  for (int r = 0; r < RC; ++r) {
-    T s = acc[r];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    acc[r] = s;
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int r = 0; r < RC; ++r)
-      if (r < rc) w[(size_t)i * ldw + r0 + r] = acc[r];
-  }
-}
-
-// Dense columns: Tnew[P[o], r] = sum_i M[i, o] W[i, r]; thread per column o,
-// rows of W staged in shared memory.  Fused curvature partials as above.
-template <typename T, int RC, int TI, int TJ>
-__global__ void __launch_bounds__(TI) dense_cols_kernel(
-    const float *__restrict__ M, int64_t ldm, int nf, int n, const int *__restrict__ P,
-    const T *__restrict__ wv, int ldw, T *__restrict__ t_out, int ldt, int R,
-    const T *__restrict__ pdot, double *__restrict__ part, const int *__restrict__ done)
-{
-  if (done && *done) return;
-  __shared__ T sw[TJ * RC];
-  __shared__ double sred[RC][TI / 32];
-  const int o = blockIdx.x * TI + threadIdx.x;
-  const int r0 = blockIdx.y * RC;
-  const int rc = min(RC, R - r0);
-  T acc[RC];
-#pragma unroll
-  for (int r = 0; r < RC; ++r) acc[r] = T(0);
-  for (int i0 = 0; i0 < nf; i0 += TJ) {
-    const int im = min(TJ, nf - i0);
-    __syncthreads();
-    for (int t = threadIdx.x; t < im * RC; t += TI) {
-      const int ii = t / RC, rr = t - ii * RC;
-      sw[t] = rr < rc ? wv[(size_t)(i0 + ii) * ldw + r0 + rr] : T(0);
-    }
-    __syncthreads();
-    if (o < n) {
-      for (int ii = 0; ii < im; ++ii) {
-        const T m = (T)__ldg(M + (size_t)(i0 + ii) * ldm + o);
-#pragma unroll
-        for (int r = 0; r < RC; ++r) acc[r] = fma(m, sw[ii * RC + r], acc[r]);
-      }
-    }
-  }
-  const int jn = o < n ? __ldg(P + o) : 0;
-  if (o < n) {
-#pragma unroll
-    for (int r = 0; r < RC; ++r)
-      if (r < rc) t_out[(size_t)jn * ldt + r0 + r] = acc[r];
-  }
-  if (part) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int r = 0; r < RC; ++r) {
-      double d = 0.0;
-      if (o < n && r < rc) d = (double)pdot[(size_t)jn * ldt + r0 + r] * (double)acc[r];
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
       if (lane == 0) sred[r][wid] = d;
     }
     __syncthreads();

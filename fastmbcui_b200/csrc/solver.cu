@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include "block.cuh"
+#include "dense.h"
 #include "factor.cuh"
 #include "factor_tc.cuh"
 #include "forces.cuh"
@@ -89,10 +90,6 @@ void rows_launch(const Solver &S, int R, const T *v, T *w, const int32_t *done, 
     dim3 grid(cdiv(S.nf, TI), cdiv(R, RC));
     mesh_rows_kernel<T, RC, TI, TJ_ROWS><<<grid, TI, 0, st>>>(S.x4(), S.n4(), S.z4(), S.nf, S.y4(), S.n, v, R,
                                                               (T)S.op.coef, w, R, R, done);
-  } else {
-    dim3 grid(cdiv(S.nf, 8), cdiv(R, RC));
-    dense_rows_kernel<T, RC><<<grid, 256, 0, st>>>(S.op.M, S.op.ldm, S.nf, S.n, S.dP(), v, R, w,
-                                                    R, R, done);
   }
 }
 
@@ -108,9 +105,6 @@ int cols_launch(const Solver &S, int R, const T *w, T *t, const T *pdot, double 
   } else if (S.op.kind == MBC_OP_MESH) {
     mesh_cols_kernel<T, RC, TI, TJ_COLS><<<grid, TI, 0, st>>>(S.x4(), S.n4(), S.z4(), S.nf, S.y4(), S.n, w, R,
                                                               (T)S.op.coef, t, R, R, pdot, part, done);
-  } else {
-    dense_cols_kernel<T, RC, TI, 32><<<grid, TI, 0, st>>>(S.op.M, S.op.ldm, S.nf, S.n, S.dP(), w, R,
-                                                          t, R, R, pdot, part, done);
   }
   return (int)grid.x;
 }
@@ -186,8 +180,9 @@ void launch_rows(const Solver &S, int R, const T *v, T *w, const int32_t *done, 
     }
     if (S.op.kind == MBC_OP_POINT_KERNEL) return p64_launch_rows(S, R, v, w, done, st);
   }
+  if (S.op.kind == MBC_OP_DENSE) return dense_launch_rows<T>(S, R, v, w, done, st);
   ++S.launches;
-  const Shape sh = pick_shape<T>(S.op.kind != MBC_OP_DENSE ? S.nf : 1 << 30, R);
+  const Shape sh = pick_shape<T>(S.nf, R);
 #define MBC_ROWS_CASE(TT, RC_, TI_) \
   if (sh.rc == RC_ && sh.ti == TI_) return rows_launch<T, RC_, TI_>(S, R, v, w, done, st);
   MBC_SHAPES(T, MBC_ROWS_CASE)
@@ -211,6 +206,7 @@ int launch_cols(const Solver &S, int R, const T *w, T *t, const T *pdot, double 
     if (use_oz(S)) return oz_launch_cols(S, R, w, t, pdot, part, done, st);
     if (S.op.kind == MBC_OP_POINT_KERNEL) return p64_launch_cols(S, R, w, t, pdot, part, done, st);
   }
+  if (S.op.kind == MBC_OP_DENSE) return dense_launch_cols<T>(S, R, w, t, pdot, part, done, st);
   ++S.launches;
   const Shape sh = pick_shape<T>(S.n, R);
 #define MBC_COLS_CASE(TT, RC_, TI_) \
@@ -224,8 +220,9 @@ int launch_cols(const Solver &S, int R, const T *w, T *t, const T *pdot, double 
 }
 
 // upper bound on the blocks of any columns-direction launch (the per-block
-// curvature partials): FP64 tiles of 16 sources or more, SIMT 64, tensor cores 128
-int cols_blocks(const Solver &S) { return p64_part_rows(S.n); }
+// curvature partials): FP64 tiles of 16 sources or more, SIMT 64, tensor cores
+// 128, dense 64 in clusters of up to 8
+int cols_blocks(const Solver &S) { return std::max(p64_part_rows(S.n), dense_part_rows(S.n)); }
 
 template void launch_rows<float>(const Solver &, int, const float *, float *, const int32_t *, cudaStream_t);
 template void launch_rows<double>(const Solver &, int, const double *, double *, const int32_t *, cudaStream_t);
