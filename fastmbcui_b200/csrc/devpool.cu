@@ -2,6 +2,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -15,52 +16,59 @@ namespace {
 constexpr int kMaxDevices = 64;
 constexpr size_t kBound = (size_t)8 << 30;  // idle bytes a pool keeps: at most this and a sixteenth of the device
 
-// One memory pool and one stream per device.  Every allocation and every
-// release is ordered on that stream and the allocating thread waits for it
-// (it is idle but for them), so memory released by one thread may go to a
-// solver of another thread and stream.
+// Idle cudaMalloc blocks of one device, by size.  (The driver's own
+// stream-ordered pools hand out kept memory as fast, but take 5 ms per GB to
+// grow, ten times cudaMalloc.)
 struct Pool {
-  std::once_flag once;
-  std::atomic<cudaMemPool_t> pool{nullptr};
-  cudaStream_t st = nullptr;
+  std::mutex mu;
+  struct Block {
+    void *ptr;
+    uint64_t seq;  // order of release: the oldest goes first when the bound is met
+  };
+  std::multimap<size_t, Block> idle;
+  size_t idle_bytes = 0, bound = 0;
+  uint64_t seq = 0;
 };
 Pool g_pools[kMaxDevices];
 std::atomic<int64_t> g_alive{0};
 
-// the pool of a device (made on first use with the device current), or NULL
-// where the device has no stream-ordered allocator
-Pool *pool_of(int dev)
+// sizes in steps of an eighth of their power of two (small) or 2 MB, so that
+// the buffers of the next pose's solver fit those of the last
+size_t rounded(size_t b)
 {
-  if (dev < 0 || dev >= kMaxDevices) return nullptr;
-  Pool &p = g_pools[dev];
-  std::call_once(p.once, [&] {
-    int ok = 0;
-    size_t free_b = 0, total_b = 0;
-    if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, dev) != cudaSuccess || !ok ||
-        cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-      cudaGetLastError();
-      return;
-    }
-    cudaMemPoolProps props{};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.handleTypes = cudaMemHandleTypeNone;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t mp = nullptr;
-    cudaStream_t st = nullptr;
-    uint64_t keep = std::min<size_t>(kBound, total_b / 16);
-    if (cudaMemPoolCreate(&mp, &props) != cudaSuccess ||
-        cudaMemPoolSetAttribute(mp, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) {
-      cudaGetLastError();
-      if (mp) cudaMemPoolDestroy(mp);
-      return;
-    }
-    p.st = st;
-    p.pool = mp;
-  });
-  return p.pool ? &p : nullptr;
+  if (b < 4096) return (b + 511) / 512 * 512;
+  if (b >= (size_t)16 << 20) return (b + ((size_t)2 << 20) - 1) / ((size_t)2 << 20) * ((size_t)2 << 20);
+  size_t step = 512;
+  while (step * 16 < b) step *= 2;
+  return (b + step - 1) / step * step;
 }
+
+// frees idle blocks, the oldest first, until at most `keep` bytes are left;
+// the pool's device is current and its mutex held
+void trim(Pool &p, size_t keep)
+{
+  while (p.idle_bytes > keep && !p.idle.empty()) {
+    auto old = p.idle.begin();
+    for (auto it = p.idle.begin(); it != p.idle.end(); ++it)
+      if (it->second.seq < old->second.seq) old = it;
+    cudaFree(old->second.ptr);
+    p.idle_bytes -= old->first;
+    p.idle.erase(old);
+  }
+}
+
+struct DeviceGuard {  // a device made current for a while
+  int prev = -1;
+  explicit DeviceGuard(int dev)
+  {
+    if (cudaGetDevice(&prev) != cudaSuccess || prev == dev) prev = -1;
+    else cudaSetDevice(dev);
+  }
+  ~DeviceGuard()
+  {
+    if (prev >= 0) cudaSetDevice(prev);
+  }
+};
 
 thread_local cudaStream_t t_stream = nullptr;
 thread_local bool t_in_call = false;
@@ -93,13 +101,18 @@ void DevMem::release()
     cudaFree(ptr);
   } else {
     Pool &p = g_pools[dev_];
-    int cur = -1;
-    if (cudaGetDevice(&cur) == cudaSuccess && cur != dev_) cudaSetDevice(dev_);
-    cudaFreeAsync(ptr, p.st);
-    if (cur >= 0 && cur != dev_) cudaSetDevice(cur);
+    DeviceGuard on(dev_);
+    std::lock_guard<std::mutex> lk(p.mu);
+    if (size_ > p.bound) {
+      cudaFree(ptr);
+    } else {
+      trim(p, p.bound - size_);
+      p.idle.emplace(size_, Pool::Block{ptr, ++p.seq});
+      p.idle_bytes += size_;
+    }
   }
   ptr = nullptr;
-  bytes = 0;
+  bytes = size_ = 0;
   dev_ = -1;
 }
 
@@ -110,25 +123,39 @@ mbc_status DevMem::reserve(size_t b)
   if (b == 0) b = 16;
   int dev = -1;
   MBC_CK(cudaGetDevice(&dev));
-  Pool *p = pooled_ ? pool_of(dev) : nullptr;
   cudaError_t e = cudaSuccess;
-  if (p) {
-    e = cudaMallocFromPoolAsync(&ptr, b, p->pool, p->st);
-    if (e == cudaErrorMemoryAllocation) {
-      // give the idle memory back and try once more
-      cudaGetLastError();
-      cudaStreamSynchronize(p->st);
-      cudaMemPoolTrimTo(p->pool, 0);
-      e = cudaMallocFromPoolAsync(&ptr, b, p->pool, p->st);
+  if (pooled_ && dev >= 0 && dev < kMaxDevices) {
+    Pool &p = g_pools[dev];
+    std::lock_guard<std::mutex> lk(p.mu);
+    if (p.bound == 0) {
+      size_t free_b = 0, total_b = 0;
+      MBC_CK(cudaMemGetInfo(&free_b, &total_b));
+      p.bound = std::min<size_t>(kBound, total_b / 16);
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(p->st);
+    size_ = rounded(b);
+    auto it = p.idle.lower_bound(size_);
+    if (it != p.idle.end() && it->first <= size_ + size_ / 8) {
+      ptr = it->second.ptr;
+      size_ = it->first;
+      p.idle_bytes -= it->first;
+      p.idle.erase(it);
+    } else {
+      e = cudaMalloc(&ptr, size_);
+      if (e == cudaErrorMemoryAllocation && !p.idle.empty()) {
+        cudaGetLastError();
+        trim(p, 0);
+        e = cudaMalloc(&ptr, size_);
+      }
+    }
     dev_ = dev;
   } else {
+    size_ = b;
     e = cudaMalloc(&ptr, b);
     dev_ = -1;
   }
   if (e != cudaSuccess) {
     ptr = nullptr;
+    size_ = 0;
     dev_ = -1;
     cudaGetLastError();
     return fail(MBC_NO_MEMORY, std::string("device allocation of ") + std::to_string(b) + " bytes: " + cudaGetErrorString(e));
@@ -139,16 +166,11 @@ mbc_status DevMem::reserve(size_t b)
 
 cudaError_t device_free_bytes(size_t *free_b, size_t *total_b)
 {
-  cudaError_t e = cudaMemGetInfo(free_b, total_b);
-  if (e != cudaSuccess) return e;
+  const cudaError_t e = cudaMemGetInfo(free_b, total_b);
   int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess) return cudaSuccess;
-  if (Pool *p = pool_of(dev)) {
-    uint64_t held = 0, used = 0;
-    if (cudaMemPoolGetAttribute(p->pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
-        cudaMemPoolGetAttribute(p->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && held > used)
-      *free_b += (size_t)(held - used);
-  }
+  if (e != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return e;
+  std::lock_guard<std::mutex> lk(g_pools[dev].mu);
+  *free_b += g_pools[dev].idle_bytes;
   return cudaSuccess;
 }
 
@@ -157,20 +179,12 @@ void pool_retain() { ++g_alive; }
 void pool_drop()
 {
   if (--g_alive != 0) return;
-  int cur = -1;
-  bool moved = false;
   for (int d = 0; d < kMaxDevices; ++d) {
-    Pool &p = g_pools[d];
-    if (!p.pool) continue;
-    if (cur < 0 && cudaGetDevice(&cur) != cudaSuccess) return;
-    if (d != cur) {
-      cudaSetDevice(d);
-      moved = true;
-    }
-    cudaStreamSynchronize(p.st);
-    cudaMemPoolTrimTo(p.pool, 0);
+    std::lock_guard<std::mutex> lk(g_pools[d].mu);
+    if (g_pools[d].idle.empty()) continue;
+    DeviceGuard on(d);
+    trim(g_pools[d], 0);
   }
-  if (moved) cudaSetDevice(cur);
 }
 
 namespace {

@@ -35,9 +35,10 @@ class CallScope {
 };
 
 // Owned device allocation that only grows; memory of the current device's
-// pool.  The pool keeps what is released up to pool_bound() bytes for the next
-// solver, gives it back to the device when an allocation of this library
-// would fail, and all of it once no plan and no solver is alive.
+// pool.  The pool keeps what is released, at most 8 GiB and a sixteenth of the
+// device, for the next solver of any thread and stream, gives it back when an
+// allocation of this library would fail, and all of it once no plan and no
+// solver is alive.
 struct DevMem {
   void *ptr = nullptr;
   size_t bytes = 0;
@@ -52,6 +53,7 @@ struct DevMem {
   void release();
 
  private:
+  size_t size_ = 0;  // of the allocation
   bool pooled_ = true;
   int dev_ = -1;  // device of the pool, -1: cudaMalloc
 };
