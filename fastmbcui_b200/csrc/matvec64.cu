@@ -35,7 +35,7 @@ Cfg pick(int M, int K, int R)
   Cfg c{};
   c.groups = (int)cdiv(R, 8 * p64::kNtMax);
   const int need = (int)cdiv(cdiv(R, c.groups), 8);
-  for (int nt : {1, 2, 3, 4, 6, 8, 10, 12})
+  for (int nt : {1, 2, 3, 4, 6, 8})
     if (nt >= need) {
       c.nt = nt;
       break;
@@ -63,7 +63,7 @@ template <int DIR, int NT, int MT, class Ker>
 void launch(const Solver &S, const p64::Args &a, const Cfg &c, int M, cudaStream_t st)
 {
   constexpr int smem = p64::smem_bytes<DIR>(NT);
-  constexpr int id = ((std::is_same<Ker, SingleLayer64>::value * 2 + DIR) * 3 + MT / 2) * 12 + NT - 1;
+  constexpr int id = ((std::is_same<Ker, SingleLayer64>::value * 2 + DIR) * 3 + MT / 2) * p64::kNtMax + NT - 1;
   if (!S.p64_smem[id]) {  // once per solver: the attribute calls cost more than a small product
     allow_max_smem(p64::pk64_kernel<DIR, NT, MT, Ker>, smem);
     S.p64_smem[id] = true;
@@ -111,9 +111,7 @@ int product(const Solver &S, int R, const double *in, double *out, double coef, 
     case 3: by_mt<DIR, 3, Ker>(S, a, c, M, st); break;
     case 4: by_mt<DIR, 4, Ker>(S, a, c, M, st); break;
     case 6: by_mt<DIR, 6, Ker>(S, a, c, M, st); break;
-    case 8: by_mt<DIR, 8, Ker>(S, a, c, M, st); break;
-    case 10: by_mt<DIR, 10, Ker>(S, a, c, M, st); break;
-    default: by_mt<DIR, 12, Ker>(S, a, c, M, st); break;
+    default: by_mt<DIR, 8, Ker>(S, a, c, M, st); break;
   }
   ++S.launches;
   if (c.parts == 1) return (int)cdiv(M, 16 * c.mt);

@@ -8,13 +8,16 @@
 // 36 to 37 TFLOP/s on the B200).  A kernel value costs 16 FP64 instructions
 // and each column one multiply-add, so a value must serve as many columns as
 // possible, and the operands of the multiply-adds must not cost issue slots.
-//   * A warp owns 16 outputs x up to 96 columns.  Each lane evaluates exactly
+//   * A warp owns 16 outputs x up to 64 columns.  Each lane evaluates exactly
 //     the four entries of its m16n8k8 A fragment in registers (rows g and
 //     g + 8, reduction positions t and t + 4, g = lane / 4, t = lane % 4), so
-//     nothing is evaluated twice inside 96 columns and no kernel value passes
+//     nothing is evaluated twice inside 64 columns and no kernel value passes
 //     through shared memory; the 16 x 8 values then meet all the warp's
-//     column tiles.  More than 96 columns: column groups (grid.y), each
-//     evaluating again, (16 + 96) / (16 + 192) of the work at 192.
+//     column tiles.  More than 64 columns: column groups (grid.y), each
+//     evaluating again.  96 columns a warp would evaluate less (7 % of the
+//     work at 192) but leave one block per SM, and evaluations and matrix
+//     instructions of too few warps to overlap: 47 % of the FP64 pipe, against
+//     73 % with two blocks (24000 points, 192 columns: 14.9 ms, against 10.8).
 //   * The vector block's tile (kKT positions x columns, FP64) is staged by
 //     cp.async two deep; its row stride is 4 modulo 16 doubles, which makes
 //     the B fragment loads free of bank conflicts.
@@ -42,7 +45,7 @@ namespace p64 {
 constexpr int kKT = 64;        // reduction positions per staged tile
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
-constexpr int kNtMax = 12;     // column tiles of 8 per warp
+constexpr int kNtMax = 8;      // column tiles of 8 per warp: two blocks per SM
 constexpr float kFar = 1e15f;  // coordinate of padded positions: finite kernel values
 
 struct Args {
@@ -60,7 +63,7 @@ struct Args {
 };
 
 __host__ __device__ constexpr int lds_for(int nt) { return nt * 8 + (nt % 2 == 0 ? 4 : 12); }
-static_assert(lds_for(12) % 16 == 4 && lds_for(3) % 16 == 4 && lds_for(1) % 16 == 4 && lds_for(8) % 16 == 4,
+static_assert(lds_for(6) % 16 == 4 && lds_for(3) % 16 == 4 && lds_for(1) % 16 == 4 && lds_for(8) % 16 == 4,
               "stride of the staged tile");
 template <int DIR>
 __host__ __device__ constexpr int coords()
@@ -89,7 +92,7 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool val
 
 // grid (output blocks of MT * 16, column groups, parts)
 template <int DIR, int NT, int MT, class Ker>
-__global__ void __launch_bounds__(kThreads, NT <= 8 ? 2 : 1) pk64_kernel(Args a)
+__global__ void __launch_bounds__(kThreads, 2) pk64_kernel(Args a)
 {
   if (a.done && *a.done) return;
   constexpr int KS = kWarps / MT;   // shares of a staged tile
