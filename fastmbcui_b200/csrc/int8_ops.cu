@@ -23,18 +23,6 @@ bool use_oz(const Solver &S)
   return S.fp64_matvec == MBC_FP64_MATVEC_INT8 && S.oz_ready && S.op.kind == MBC_OP_POINT_KERNEL;
 }
 
-// dst[k, c] = src[idx[k], c] (K x R, FP64): the vector block in the order the
-// planes' reduction axis walks
-__global__ void oz_gather_kernel(int K, int R, const int32_t *__restrict__ idx, const double *__restrict__ src,
-                                 double *__restrict__ dst, const int32_t *__restrict__ done)
-{
-  if (done && *done) return;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)K * R) return;
-  const int k = (int)(t / R), c = (int)(t - (int64_t)k * R);
-  dst[t] = src[(size_t)idx[k] * R + c];
-}
-
 // the coordinates each direction's digit kernel reads: (rows, normals,
 // sources) with the reduction axis in Morton order
 static void oz_coords(const Solver &S, int DIR, const float4 **xr, const float4 **nr, const float4 **ys)
@@ -71,17 +59,13 @@ static int oz_launch(const Solver &S, int R, const double *vin, double *out, con
   const int M = DIR == 0 ? S.nf : S.n;
   const int K = DIR == 0 ? S.n : S.nf;
   const int np = oz::np_for(R), groups = oz::groups_for(R);
-  if (S.m_oz_b.bytes < oz::bimg_bytes(K, R) || S.m_oz_bexp.bytes < sizeof(int32_t) * oz::bexp_count(K, R) ||
-      S.m_oz_v.bytes < sizeof(double) * (size_t)K * R) {
+  if (S.m_oz_b.bytes < oz::bimg_bytes(K, R) || S.m_oz_bexp.bytes < sizeof(int32_t) * oz::bexp_count(K, R)) {
     S.oz_unprepared = true;
     return 0;
   }
-  double *vg = (double *)S.m_oz_v.ptr;
-  oz_gather_kernel<<<(unsigned)cdiv((int64_t)K * R, 256), 256, 0, st>>>(K, R, (const int32_t *)S.m_oz_q[DIR].ptr,
-                                                                       vin, vg, done);
-  oz::oz_pack_b_kernel<<<dim3(oz::nchunks_for(K), groups), 512, 0, st>>>(
-      vg, K, R, np, (int8_t *)S.m_oz_b.ptr, S.m_oz_b.bytes, (int32_t *)S.m_oz_bexp.ptr,
-      S.m_oz_bexp.bytes / sizeof(int32_t), done, (int32_t *)S.m_err.ptr);
+  oz::oz_pack_b_kernel<<<dim3(oz::nchunks_for(K) * oz::kPackCtas, groups), 512, 0, st>>>(
+      vin, (const int32_t *)S.m_oz_q[DIR].ptr, K, R, np, (int8_t *)S.m_oz_b.ptr, S.m_oz_b.bytes,
+      (int32_t *)S.m_oz_bexp.ptr, S.m_oz_bexp.bytes / sizeof(int32_t), done, (int32_t *)S.m_err.ptr);
   oz::OzArgs a{};
   const DevMem &planes = S.oz_slab ? S.m_oz_a[0] : S.m_oz_a[DIR];
   a.adig = (const int8_t *)planes.ptr;
@@ -118,14 +102,13 @@ static int oz_launch(const Solver &S, int R, const double *vin, double *out, con
   const int tiles = oz::row_tiles(M);
   if (!S.oz_slab) {
     mma(0, tiles);
-    S.launches += 3;
+    S.launches += 2;
   } else {
     // the planes of each slab of rows, then its products
     const int per = S.oz_slab_tiles[DIR];
     const size_t smem = (DIR == 0 ? 1 : 2) * sizeof(float4) * oz::kChunk;
     const float4 *cx, *cn, *cy;
     oz_coords(S, DIR, &cx, &cn, &cy);
-    ++S.launches;  // the gather
     for (int r0 = 0; r0 < tiles; r0 += per) {
       const int cnt = std::min(per, tiles - r0);
       oz::oz_digits_kernel<DIR><<<dim3(oz::nchunks_for(K), cnt), 256, smem, st>>>(
@@ -247,13 +230,11 @@ mbc_status mbc::Solver::ensure_oz(cudaStream_t st, int R)
     const int K = std::max(n, nf);
     MBC_TRY(m_oz_b.reserve(oz::bimg_bytes(K, std::max(R, 1))));
     MBC_TRY(m_oz_bexp.reserve(sizeof(int32_t) * oz::bexp_count(K, std::max(R, 1))));
-    MBC_TRY(m_oz_v.reserve(sizeof(double) * (size_t)K * std::max(R, 1)));
     MBC_TRY(oz_selfcheck(st));
   }
   const int K = std::max(n, nf);
   MBC_TRY(m_oz_b.reserve(oz::bimg_bytes(K, R)));
   MBC_TRY(m_oz_bexp.reserve(sizeof(int32_t) * oz::bexp_count(K, R)));
-  MBC_TRY(m_oz_v.reserve(sizeof(double) * (size_t)K * R));
   return MBC_OK;
 }
 

@@ -62,6 +62,7 @@
 // copies, free tensor memory, return).
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -334,39 +335,55 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const float4 *__restrict
 }
 
 // ---------------------------------------------------------------------------
-// B image of the input block vin (K x R, row-major FP64) for one matvec.
-// Grid (chunks, groups), 512 threads.  Layout: bimg[(grp * nks + ks) *
+// B image of the input block vin (R columns, row-major FP64; the k-th
+// position of the reduction axis is row idx[k]) for one matvec.  A cluster of
+// kPackCtas blocks per (chunk, column group): each takes kChunkSteps /
+// kPackCtas k-steps, finds its columns' maxima, and the cluster combines them
+// through distributed shared memory before the digits are written; grid
+// (chunks * kPackCtas, groups), 512 threads.  Layout: bimg[(grp * nks + ks) *
 // bstage_bytes(np) + ...], rows p * np + r (plane p, column grp * np + r) of
 // the swizzled image; bexp[(grp * nchunks + c) * np + r].
-__global__ void __launch_bounds__(512) oz_pack_b_kernel(const double *__restrict__ vin, int K, int R,
-                                                        int np, int8_t *__restrict__ bimg, size_t bimg_size,
-                                                        int32_t *__restrict__ bexp, size_t bexp_size,
-                                                        const int32_t *__restrict__ done,
-                                                        int32_t *__restrict__ err)
+// What bounds it: launch and memory latency (7 M values at 48000 x 144).  One
+// block per chunk left 48 of 148 SMs working, after a pass that wrote the block
+// in the axis' order.
+constexpr int kPackCtas = 8;
+constexpr int kPackSteps = kChunkSteps / kPackCtas;
+static __global__ void __cluster_dims__(kPackCtas, 1, 1) __launch_bounds__(512)
+    oz_pack_b_kernel(const double *__restrict__ vin, const int32_t *__restrict__ idx, int K, int R, int np,
+                     int8_t *__restrict__ bimg, size_t bimg_size, int32_t *__restrict__ bexp, size_t bexp_size,
+                     const int32_t *__restrict__ done, int32_t *__restrict__ err)
 {
   if (done && *done) return;
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
   __shared__ double s_max[16][kNpMax];
+  __shared__ double s_own[kNpMax];
   __shared__ int s_exp[kNpMax];
-  const int c = blockIdx.x, grp = blockIdx.y;
+  __shared__ int s_idx[kPackSteps * kKS];
+  const int c = blockIdx.x / kPackCtas, part = blockIdx.x % kPackCtas, grp = blockIdx.y;
   const int nks = nks_for(K);
   const int nchunks = nchunks_for(K);
-  const int ks0 = c * kChunkSteps;
-  const int ks1 = min(ks0 + kChunkSteps, nks);
+  const int ks0 = c * kChunkSteps + part * kPackSteps;
+  const int ks1 = min(ks0 + kPackSteps, nks);
   const int kbase = ks0 * kKS;
-  const int kcount = min(kChunk, K - kbase);
+  const int kcount = max(0, min(kPackSteps * kKS, K - kbase));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // pass 1: column maxima over the chunk (warp w takes rows w, w + 16, ...)
+  for (int k = threadIdx.x; k < kcount; k += blockDim.x) s_idx[k] = idx[kbase + k];
+  __syncthreads();
+  // pass 1: column maxima over the block's rows (warp w takes rows w, w + 16, ...)
   for (int cb = 0; cb < np; cb += 32) {
     const int col = cb + lane;
     const int gc = grp * np + col;
     double m = 0.0;
     bool finite = true;
-    if (col < np && gc < R)
+    if (col < np && gc < R) {
+#pragma unroll 4
       for (int k = warp; k < kcount; k += 16) {
-        const double x = vin[(size_t)(kbase + k) * R + gc];
+        const double x = vin[(size_t)s_idx[k] * R + gc];
         finite = finite && isfinite(x);
         m = fmax(m, fabs(x));
       }
+    }
     if (col < np) s_max[warp][col] = finite ? m : __longlong_as_double(0x7FF0000000000000ll);
   }
   __syncthreads();
@@ -374,15 +391,24 @@ __global__ void __launch_bounds__(512) oz_pack_b_kernel(const double *__restrict
     double m = 0.0;
 #pragma unroll
     for (int w = 0; w < 16; ++w) m = fmax(m, s_max[w][col]);
+    s_own[col] = m;
+  }
+  cl.sync();
+  for (int col = threadIdx.x; col < np; col += blockDim.x) {
+    double m = 0.0;
+#pragma unroll
+    for (int r = 0; r < kPackCtas; ++r) m = fmax(m, *cl.map_shared_rank(&s_own[col], r));
     const int e = isfinite(m) ? ceil_exp2(m) : kNonFinite;
     s_exp[col] = e;
-    const size_t ei = bexp_index(grp, c, col, nchunks, np);
-    if (ei < bexp_size) bexp[ei] = e;
-    else atomicMax(err, 4);
+    if (part == 0) {
+      const size_t ei = bexp_index(grp, c, col, nchunks, np);
+      if (ei < bexp_size) bexp[ei] = e;
+      else atomicMax(err, 4);
+    }
   }
-  __syncthreads();
+  cl.sync();  // the maxima are read; s_exp is complete
   // pass 2: units (k-step, column, 16-byte group); lanes run over columns
-  const int units = (ks1 - ks0) * np * 8;
+  const int units = max(0, ks1 - ks0) * np * 8;
   for (int t = threadIdx.x; t < units; t += blockDim.x) {
     const int col = t % np;
     const int rest = t / np;
@@ -397,7 +423,7 @@ __global__ void __launch_bounds__(512) oz_pack_b_kernel(const double *__restrict
     for (int e = 0; e < 16; ++e) {
       const int k = kk0 + e;
       uint64_t tb = 0;
-      if (gc < R && k < kcount) tb = digit_bytes(vin[(size_t)(kbase + k) * R + gc], s_exp[col]);
+      if (gc < R && k < kcount) tb = digit_bytes(vin[(size_t)s_idx[k] * R + gc], s_exp[col]);
 #pragma unroll
       for (int p = 0; p < kDigits; ++p)
         w[p][e >> 2] |= (uint32_t)((tb >> (8 * (kDigits - 1 - p))) & 0xFFu) << (8 * (e & 3));
