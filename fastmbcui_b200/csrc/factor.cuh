@@ -1,7 +1,9 @@
 // Supernodal KL factor, one CTA per supernode s:
 //   1. Theta_s = K(:, I_s)^T K(:, I_s) over all nf collocation rows, written
 //      in reversed order, column-major (kl_chol.cu:166-223); the K panels are
-//      generated tile by tile in shared memory and never stored;
+//      generated tile by tile in shared memory and never stored (sets of at
+//      most 64 entries: by gram_kernel, larger FP32 ones by gram_tc_kernel
+//      beforehand, so that this kernel only loads Theta_s);
 //   2. Theta_rev = U^T U in place, U in the upper triangle (kl_chol.cu:16-36),
 //      right-looking so each step is a parallel rank-1 update;
 //   3. every column c of s: L(:,c) = reverse(U_nb^-1 e_nb) on the leading
@@ -38,9 +40,13 @@ struct FactorArgs {
   // has cancelled most of its digits: the supernode is flagged for the FP64
   // retry (FP32 launches); 0 flags only non-positive pivots.
   double pivot_tol;
-  // 1: Theta_s of every supernode of the launch is already in the global
-  // Theta array (gram_tc_kernel, FP32 launches): step 1 only loads it
+  // 1: Theta_s of every supernode of the launch is already in global memory
+  // (gram_kernel, gram_tc_kernel): step 1 only loads it, the sum in order of
+  // gram_parts copies gram_stride entries apart
   int32_t gram_ready;
+  const void *gram_src;
+  int32_t gram_parts;
+  int64_t gram_stride;
   int32_t smem_cap;  // largest n_s kept in shared memory
   int32_t tile_rows; // panel rows per tile
   int32_t *bad_list, *bad_count;
@@ -102,10 +108,14 @@ __global__ void __launch_bounds__(NT) factor_kernel(FactorArgs a, T *__restrict_
   __syncthreads();
 
   // 1. Gram assembly, entry chunks of NT*EPT upper-triangle entries (or,
-  // with gram_ready, the tensor-core Gram from the global slice)
+  // with gram_ready, the sum of the parts in global memory)
   if (a.gram_ready && in_smem) {
-    const T *src = theta + a.th_ptr[s];
-    for (int e = tid; e < ns * ns; e += NT) A[e] = src[e];
+    const T *src = reinterpret_cast<const T *>(a.gram_src) + a.th_ptr[s];
+    for (int e = tid; e < ns * ns; e += NT) {
+      T v = src[e];
+      for (int q = 1; q < a.gram_parts; ++q) v += src[(size_t)q * a.gram_stride + e];
+      A[e] = v;
+    }
   }
   for (int e0 = 0; e0 < (a.gram_ready ? 0 : ne); e0 += NT * EPT) {
     int pe[EPT], qe[EPT];

@@ -18,6 +18,7 @@
 #include "factor.cuh"
 #include "factor_tc.cuh"
 #include "forces.cuh"
+#include "gram.cuh"
 #include "matvec.cuh"
 #include "matvec64.h"
 #include "matvec_mesh.cuh"
@@ -303,16 +304,110 @@ static mbc_status launch_gram(Solver &S, const std::vector<int32_t> &gram, float
   return MBC_OK;
 }
 
-// Launch the factor kernels over the given per-class supernode lists.  In
-// FP32 the supernodes with tiles.tc_min_ns <= n_s <= ftc::kMaxNs take their
-// Gram from the tensor cores first (tc_min_ns = 0: none).
+// the operator, the plan and the set arrays of a factor launch
+static FactorArgs factor_args(const Solver &S)
+{
+  FactorArgs a{};
+  a.sup_ptr = S.d_sup_ptr();
+  a.sup_ind = S.d_sup_ind();
+  a.set_ptr = S.d_set_ptr();
+  a.set_ind = S.d_set_ind();
+  a.lptr = S.d_lptr();
+  a.th_ptr = S.d_th_ptr();
+  a.kind = S.op.kind;
+  a.xr = S.x4();
+  a.nr = S.n4();
+  a.zr = S.z4();
+  a.ys = S.y4();
+  a.M = S.op.M;
+  a.ldm = S.op.ldm;
+  a.Pinv = S.d_Pinv();
+  a.nf = S.nf;
+  a.coef = S.op.coef;
+  return a;
+}
+
+// Theta of supernodes with at most gram::kMaxNs entries by gram_kernel: one
+// launch per kernel shape.  The rows are cut into as many parts as give about
+// four blocks per SM (at least four panels each, at most half a GB of copies);
+// *src, *parts and *stride are where factor_kernel finds the copies.
+template <typename T>
+static mbc_status launch_grams(Solver &S, const std::vector<int32_t> &ids, T *theta, const void **src, int *parts,
+                               int64_t *stride, cudaStream_t st)
+{
+  const Plan &p = *S.plan;
+  const int64_t th_n = p.th_ptr.back();
+  int64_t np = cdiv(4 * 148, (int64_t)ids.size());
+  np = std::min<int64_t>(np, std::max(1, S.nf / 512));
+  np = std::min<int64_t>(np, ((int64_t)512 << 20) / std::max<int64_t>(1, th_n * (int64_t)sizeof(T)));
+  np = std::max<int64_t>(1, std::min<int64_t>(np, gram::kMaxParts));
+  T *dst = theta;
+  if (np > 1) {
+    MBC_TRY(S.gram_part.reserve((size_t)np * th_n * sizeof(T)));
+    dst = (T *)S.gram_part.ptr;
+  }
+  *src = dst;
+  *parts = (int)np;
+  *stride = th_n;
+  // shapes: FP32 up to 32 and 64 entries, FP64 one per 16
+  constexpr int kShapes = sizeof(T) == 4 ? 2 : 4, kStep = gram::kMaxNs / kShapes;
+  std::vector<int32_t> by[kShapes], all;
+  for (int32_t s : ids) by[(p.set_ptr[s + 1] - p.set_ptr[s] - 1) / kStep].push_back(s);
+  for (auto &v : by) {
+    std::stable_sort(v.begin(), v.end(), [&](int32_t a, int32_t b) {
+      return p.set_ptr[a + 1] - p.set_ptr[a] > p.set_ptr[b + 1] - p.set_ptr[b];
+    });
+    all.insert(all.end(), v.begin(), v.end());
+  }
+  MBC_TRY(upload(S.gram_ids, all, st));
+  size_t at = all.size();
+  for (int k = kShapes - 1; k >= 0; --k) {  // the largest sets first
+    at -= by[k].size();
+    if (by[k].empty()) continue;
+    const int ns_max = (k + 1) * kStep;
+    gram::Args a{};
+    a.f = factor_args(S);
+    a.f.list = (const int32_t *)S.gram_ids.ptr + at;
+    a.f.count = (int32_t)by[k].size();
+    a.parts = (int)np;
+    a.part_stride = th_n;
+    a.rows = gram::rows_for<T>(ns_max);
+    a.ld = gram::ld_for<T>(ns_max);
+    const int smem = gram::smem_bytes<T>(ns_max);
+    const dim3 grid((unsigned)by[k].size(), (unsigned)np);
+    auto go = [&](auto kern) -> mbc_status {
+      MBC_TRY(allow_max_smem(kern, smem));
+      kern<<<grid, gram::kThreads, smem, st>>>(a, dst);
+      return MBC_OK;
+    };
+    if constexpr (sizeof(T) == 4) {
+      MBC_TRY(go(gram::gram_kernel<T, 1>));
+    } else {
+      switch (k) {
+        case 0: MBC_TRY(go(gram::gram_kernel<T, 1>)); break;
+        case 1: MBC_TRY(go(gram::gram_kernel<T, 2>)); break;
+        case 2: MBC_TRY(go(gram::gram_kernel<T, 3>)); break;
+        default: MBC_TRY(go(gram::gram_kernel<T, 4>)); break;
+      }
+    }
+    ++S.launches;
+    MBC_CKL();
+  }
+  return MBC_OK;
+}
+
+// Launch the factor kernels over the given per-class supernode lists.  Theta
+// of the sets with at most gram::kMaxNs entries comes from gram_kernel, in
+// FP32 that of the larger ones up to ftc::kMaxNs (and of all from
+// tiles.tc_min_ns on; 0: none) from the tensor cores; factor_kernel forms the
+// others itself.
 template <typename T, typename LT>
 static mbc_status run_factor(Solver &S, const std::vector<int32_t> *lists, T *theta, LT *lval,
                              double shift, double pivot_tol, int32_t *d_bad_list,
                              int32_t *d_bad_count, cudaStream_t st)
 {
   const Plan &p = *S.plan;
-  std::vector<int32_t> simt[4], tcl[4], gram;
+  std::vector<int32_t> simt[4], tcl[4], grl[4], gram, small;
   const int tc_min = std::is_same<T, float>::value ? S.tiles.tc_min_ns : 0;
   for (int c = 0; c < 4; ++c)
     for (int32_t s : lists[c]) {
@@ -320,42 +415,36 @@ static mbc_status run_factor(Solver &S, const std::vector<int32_t> *lists, T *th
       if (tc_min > 0 && ns >= tc_min && ns <= ftc::kMaxNs) {
         tcl[c].push_back(s);
         gram.push_back(s);
+      } else if (c < 3 && ns <= gram::kMaxNs) {
+        grl[c].push_back(s);
+        small.push_back(s);
       } else {
         simt[c].push_back(s);
       }
     }
   if constexpr (std::is_same<T, float>::value)
     if (!gram.empty()) MBC_TRY(launch_gram(S, gram, theta, st));
-  for (int job = 0; job < 8; ++job) {
-    const int c = job & 3, ready = job >> 2;
-    const auto &lst = ready ? tcl[c] : simt[c];
+  const void *gram_src = nullptr;
+  int gram_parts = 1;
+  int64_t gram_stride = 0;
+  if (!small.empty()) MBC_TRY(launch_grams<T>(S, small, theta, &gram_src, &gram_parts, &gram_stride, st));
+  for (int job = 0; job < 12; ++job) {
+    const int c = job & 3, from = job >> 2;  // Theta: 0 factor_kernel's own, 1 tensor cores, 2 gram_kernel
+    const auto &lst = from == 0 ? simt[c] : from == 1 ? tcl[c] : grl[c];
     if (lst.empty()) continue;
-    DevMem &dl = ready ? S.class_list_tc[c] : S.class_list[c];
+    DevMem &dl = from == 0 ? S.class_list[c] : from == 1 ? S.class_list_tc[c] : S.class_list_gr[c];
     MBC_TRY(upload(dl, lst, st));
     int ns_max = 0;
     for (int32_t s : lst) ns_max = std::max(ns_max, p.set_ptr[s + 1] - p.set_ptr[s]);
-    FactorArgs a{};
+    FactorArgs a = factor_args(S);
     a.list = (const int32_t *)dl.ptr;
     a.count = (int32_t)lst.size();
-    a.sup_ptr = S.d_sup_ptr();
-    a.sup_ind = S.d_sup_ind();
-    a.set_ptr = S.d_set_ptr();
-    a.set_ind = S.d_set_ind();
-    a.lptr = S.d_lptr();
-    a.th_ptr = S.d_th_ptr();
-    a.kind = S.op.kind;
-    a.xr = S.x4();
-    a.nr = S.n4();
-    a.zr = S.z4();
-    a.ys = S.y4();
-    a.M = S.op.M;
-    a.ldm = S.op.ldm;
-    a.Pinv = S.d_Pinv();
-    a.nf = S.nf;
-    a.coef = S.op.coef;
     a.shift = shift;
     a.pivot_tol = pivot_tol;
-    a.gram_ready = ready;
+    a.gram_ready = from != 0;
+    a.gram_src = from == 2 ? gram_src : theta;
+    a.gram_parts = from == 2 ? gram_parts : 1;
+    a.gram_stride = gram_stride;
     a.bad_list = d_bad_list;
     a.bad_count = d_bad_count;
     const int nt = kClassThreads[c];

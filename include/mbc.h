@@ -159,7 +159,9 @@ mbc_status mbc_solver_get_factor(const mbc_solver *s, double *lval_host, double 
  * (256), <= max_ns[2] (512), each with Theta_s in shared memory, and larger
  * ones (512 threads, Theta_s in global memory).  tile_rows[c] is how many
  * collocation rows of the K panel a class stages per pass (class 3, and any
- * class whose shared memory would not fit, use at most that many).  The
+ * class whose shared memory would not fit, use at most that many); sets of
+ * at most 64 entries in the first three classes form Theta_s in a kernel of
+ * fixed 64- or 128-row panels before their class kernel factors it.  The
  * shapes change the order of the Gram sums (results agree to rounding), not
  * the method.  In FP32 factors, supernodes with tc_min_ns <= n_s <= 192 form
  * Theta_s on the tensor cores (tcgen05, 3xTF32 with FP32 chunk sums) before
