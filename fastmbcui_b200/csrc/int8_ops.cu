@@ -106,7 +106,7 @@ static int oz_launch(const Solver &S, int R, const double *vin, double *out, con
   } else {
     // the planes of each slab of rows, then its products
     const int per = S.oz_slab_tiles[DIR];
-    const size_t smem = (DIR == 0 ? 1 : 2) * sizeof(float4) * oz::kChunk;
+    const size_t smem = oz::digits_smem(DIR);
     const float4 *cx, *cn, *cy;
     oz_coords(S, DIR, &cx, &cn, &cy);
     for (int r0 = 0; r0 < tiles; r0 += per) {
@@ -147,7 +147,7 @@ mbc_status mbc::Solver::ensure_oz(cudaStream_t st, int R)
     MBC_CK(device_free_bytes(&free_b, &total_b));
     MBC_TRY(m_oz_aexp[0].reserve(sizeof(int32_t) * oz::aexp_count(nf, n)));
     MBC_TRY(m_oz_aexp[1].reserve(sizeof(int32_t) * oz::aexp_count(n, nf)));
-    const size_t sm0 = sizeof(float4) * oz::kChunk, sm1 = 2 * sizeof(float4) * oz::kChunk;
+    const size_t sm0 = oz::digits_smem(0), sm1 = oz::digits_smem(1);
     MBC_TRY(allow_max_smem(oz::oz_digits_kernel<0>, sm0));
     MBC_TRY(allow_max_smem(oz::oz_digits_kernel<1>, sm1));
     MBC_TRY(oz_allow<8>());

@@ -1,6 +1,4 @@
 // Dispatch of the FP64 point-kernel products (matvec64.cuh).
-#include <algorithm>
-#include <cmath>
 #include <type_traits>
 
 #include <cuda_runtime.h>
@@ -14,71 +12,51 @@ namespace mbc {
 
 namespace {
 
-constexpr double kSMs = 148.0;
-constexpr size_t kPartsBytes = (size_t)64 << 20;  // most that the partial blocks of a split may take
-
 struct Cfg {
-  int nt, groups, mt, parts;
+  int nt, groups, z;
 };
 
-// The split of an M x K product over R columns.  Blocks of one SM share its
-// FP64 pipe, so a launch lasts as long as the SM with the most blocks:
-// ceil(blocks parts / 148) blocks of 16 mt K / parts entries at 16 + 8 nt
-// FP64 multiply-adds each, plus ~2 us a block to start and to sum its shares,
-// and no shorter than its reads of the vector block from L2 (~6 TB/s).
-// Splitting the reduction (parts > 1) costs a second kernel and the partial
-// blocks' round trip.  The shape with the smallest estimate is taken: at
-// R = 12 and 3000 points 16 outputs per block and no split, at R = 60 and
-// 20000 points 64 outputs and a split that fills the last wave.
+// The split of an M x K product over R columns: the fewest column groups of at
+// most 64, and the smallest cluster (1, 2, 4, 8 blocks along the reduction)
+// that gives a thousand blocks, seven per SM: fewer leave SMs idle or a last
+// wave short, larger clusters cost more to start and to add up.  Measured
+// (B200, us of K; clusters of 1 / 2 / 4 / 8): 3000 x 3000, 12 columns 123 / 82 /
+// 75 / 71; 20000, 60 columns 3351 / 2716 / 2432 / 2669; 32000, 96 columns
+// 10666 / 10564 / 10913 / 11651.
 Cfg pick(int M, int K, int R)
 {
   Cfg c{};
   c.groups = (int)cdiv(R, 8 * p64::kNtMax);
   const int need = (int)cdiv(cdiv(R, c.groups), 8);
-  for (int nt : {1, 2, 3, 4, 6, 8})
-    if (nt >= need) {
-      c.nt = nt;
-      break;
-    }
-  const double np = 8.0 * c.nt, rate = 64.0 * 1.8e3;  // multiply-adds per us and SM
-  double best = 1e300;
-  for (int mt : {4, 2, 1})
-    for (int parts = 1; parts <= 8; ++parts) {
-      if (parts > 1 && ((size_t)parts * M * R * sizeof(double) > kPartsBytes || (int)cdiv(K, p64::kKT) < 4 * parts)) break;
-      const double blocks = (double)cdiv(M, 16 * mt) * c.groups;
-      const double work = 16.0 * mt * K * (16.0 + np) / rate / parts;
-      const double l2 = blocks * K * np * 8.0 / 6e6;
-      double t = std::max(std::ceil(blocks * parts / kSMs) * (work + 2.0), l2);
-      if (parts > 1) t += 4.0 + 2.0 * parts * (double)M * R * 8.0 / 5e6;
-      if (t < 0.98 * best) {
-        best = t;
-        c.mt = mt;
-        c.parts = parts;
-      }
-    }
+  c.nt = need == 5 ? 6 : need == 7 ? 8 : need;
+  const int64_t blocks = (int64_t)cdiv(M, p64::kRows) * c.groups;
+  for (c.z = 1; c.z < 8 && blocks * c.z < 1000 && (int)cdiv(K, p64::kKT) >= 4 * c.z; c.z *= 2) {
+  }
   return c;
 }
 
-template <int DIR, int NT, int MT, class Ker>
+template <int DIR, int NT, class Ker>
 void launch(const Solver &S, const p64::Args &a, const Cfg &c, int M, cudaStream_t st)
 {
   constexpr int smem = p64::smem_bytes<DIR>(NT);
-  constexpr int id = ((std::is_same<Ker, SingleLayer64>::value * 2 + DIR) * 3 + MT / 2) * p64::kNtMax + NT - 1;
+  constexpr int id = (std::is_same<Ker, SingleLayer64>::value * 2 + DIR) * p64::kNtMax + NT - 1;
   if (!S.p64_smem[id]) {  // once per solver: the attribute calls cost more than a small product
-    allow_max_smem(p64::pk64_kernel<DIR, NT, MT, Ker>, smem);
+    allow_max_smem(p64::pk64_kernel<DIR, NT, Ker>, smem);
     S.p64_smem[id] = true;
   }
-  p64::pk64_kernel<DIR, NT, MT, Ker><<<dim3(cdiv(M, 16 * MT), c.groups, c.parts), p64::kThreads, smem, st>>>(a);
-}
-
-template <int DIR, int NT, class Ker>
-void by_mt(const Solver &S, const p64::Args &a, const Cfg &c, int M, cudaStream_t st)
-{
-  switch (c.mt) {
-    case 4: launch<DIR, NT, 4, Ker>(S, a, c, M, st); break;
-    case 2: launch<DIR, NT, 2, Ker>(S, a, c, M, st); break;
-    default: launch<DIR, NT, 1, Ker>(S, a, c, M, st); break;
-  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(cdiv(M, p64::kRows), c.groups, c.z);
+  cfg.blockDim = dim3(p64::kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = c.z;
+  cfg.attrs = at;
+  cfg.numAttrs = c.z > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, p64::pk64_kernel<DIR, NT, Ker>, a);  // an error stays pending for the caller's check
 }
 
 // the product; returns the rows of the curvature partials
@@ -87,8 +65,7 @@ int product(const Solver &S, int R, const double *in, double *out, double coef, 
             const int32_t *done, cudaStream_t st)
 {
   const int M = DIR == 0 ? S.nf : S.n, K = DIR == 0 ? S.n : S.nf;
-  Cfg c = pick(M, K, R);
-  if (c.parts > 1 && S.m_p64.reserve((size_t)c.parts * M * R * sizeof(double)) != MBC_OK) c.parts = 1;
+  const Cfg c = pick(M, K, R);
   p64::Args a{};
   a.xr = S.x4();
   a.nr = S.n4();
@@ -97,8 +74,6 @@ int product(const Solver &S, int R, const double *in, double *out, double coef, 
   a.n = S.n;
   a.in = in;
   a.out = out;
-  a.parts = (double *)S.m_p64.ptr;
-  a.nparts = c.parts;
   a.R = R;
   a.groups = c.groups;
   a.coef = coef;
@@ -106,34 +81,18 @@ int product(const Solver &S, int R, const double *in, double *out, double coef, 
   a.part = part;
   a.done = done;
   switch (c.nt) {
-    case 1: by_mt<DIR, 1, Ker>(S, a, c, M, st); break;
-    case 2: by_mt<DIR, 2, Ker>(S, a, c, M, st); break;
-    case 3: by_mt<DIR, 3, Ker>(S, a, c, M, st); break;
-    case 4: by_mt<DIR, 4, Ker>(S, a, c, M, st); break;
-    case 6: by_mt<DIR, 6, Ker>(S, a, c, M, st); break;
-    default: by_mt<DIR, 8, Ker>(S, a, c, M, st); break;
+    case 1: launch<DIR, 1, Ker>(S, a, c, M, st); break;
+    case 2: launch<DIR, 2, Ker>(S, a, c, M, st); break;
+    case 3: launch<DIR, 3, Ker>(S, a, c, M, st); break;
+    case 4: launch<DIR, 4, Ker>(S, a, c, M, st); break;
+    case 6: launch<DIR, 6, Ker>(S, a, c, M, st); break;
+    default: launch<DIR, 8, Ker>(S, a, c, M, st); break;
   }
   ++S.launches;
-  if (c.parts == 1) return (int)cdiv(M, 16 * c.mt);
-  const unsigned blocks = cdiv(M, p64::kSumRows);
-  p64::pk64_sum_kernel<<<blocks, 256, 0, st>>>(M, R, c.parts, a.parts, coef, out, pdot, part, done);
-  ++S.launches;
-  return (int)blocks;
+  return (int)cdiv(M, p64::kRows) * c.z;
 }
 
 }  // namespace
-
-mbc_status p64_reserve(const Solver &S, int R)
-{
-  if (S.op.kind != MBC_OP_POINT_KERNEL) return MBC_OK;
-  size_t b = 0;
-  for (int dir = 0; dir < 2; ++dir) {
-    const int M = dir == 0 ? S.nf : S.n, K = dir == 0 ? S.n : S.nf;
-    const Cfg c = pick(M, K, R);
-    if (c.parts > 1) b = std::max(b, (size_t)c.parts * M * R * sizeof(double));
-  }
-  return b ? S.m_p64.reserve(b) : MBC_OK;
-}
 
 void p64_launch_rows(const Solver &S, int R, const double *v, double *w, const int32_t *done, cudaStream_t st)
 {

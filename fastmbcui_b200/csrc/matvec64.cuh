@@ -21,19 +21,21 @@
 //   * The vector block's tile (kKT positions x columns, FP64) is staged by
 //     cp.async two deep; its row stride is 4 modulo 16 doubles, which makes
 //     the B fragment loads free of bank conflicts.
-//   * A block is 8 warps: MT tiles of 16 outputs x KS = 8 / MT shares of every
-//     staged tile.  Small scenes take MT = 1 (16 outputs per block: 188 blocks
-//     at 3000 points), large ones 64 outputs, where the tile is read from L2
-//     less often.  The shares of a tile are summed through shared memory at
-//     the end, and with `parts` > 1 the reduction axis is further cut over
-//     grid.z into partial blocks that pk64_sum_kernel adds in order, so that
-//     the last wave is full at every size.  All sums have a fixed order.
+//   * A block is 8 warps: kMT = 4 tiles of 16 outputs x KS = 2 shares of every
+//     staged tile (16 or 32 outputs a block, with more shares, read the tiles
+//     from L2 more often and sum more: 10 to 40 % slower at every size but the
+//     smallest).  The shares of a tile are summed through shared memory at the
+//     end.  Where blocks are too few, or fill a last wave badly, the
+//     reduction axis is further cut over a cluster of up to 8 blocks, which add
+//     their results through distributed shared memory.  All sums have a fixed
+//     order.
 // Positions past the end carry a far-away point and zero vector entries.
 // Measured (B200, K then K^T): 20000 x 20000, 60 columns 4.76 ms, against
 // 10.92 ms for one thread per output with FP64 FMAs and one evaluation per 32
 // columns; the FP64 pipe's floor is 3.3 ms.
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -45,6 +47,8 @@ namespace p64 {
 constexpr int kKT = 64;        // reduction positions per staged tile
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
+constexpr int kMT = 4;         // tiles of 16 outputs per block
+constexpr int kRows = 16 * kMT;
 constexpr int kNtMax = 8;      // column tiles of 8 per warp: two blocks per SM
 constexpr float kFar = 1e15f;  // coordinate of padded positions: finite kernel values
 
@@ -54,11 +58,10 @@ struct Args {
   int nf, n;
   const double *in;       // K x R vector block (row stride R)
   double *out;            // M x R
-  double *parts;          // nparts > 1: [part][M][R] partial sums (without coef)
-  int nparts, R, groups;
+  int R, groups;
   double coef;
-  const double *pdot;     // curvature partials (nparts == 1): p, M x R, or NULL
-  double *part;           // per block of outputs: part[blockIdx.x * R + r]
+  const double *pdot;     // curvature partials: p, M x R, or NULL
+  double *part;           // per slice of outputs: part[(blockIdx.x * cluster size + rank) * R + r]
   const int32_t *done;
 };
 
@@ -90,11 +93,12 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool val
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(s), "l"(gmem), "r"(valid ? 8 : 0) : "memory");
 }
 
-// grid (output blocks of MT * 16, column groups, parts)
-template <int DIR, int NT, int MT, class Ker>
+// grid (output blocks of kRows, column groups, cluster size)
+template <int DIR, int NT, class Ker>
 __global__ void __launch_bounds__(kThreads, 2) pk64_kernel(Args a)
 {
   if (a.done && *a.done) return;
+  constexpr int MT = kMT;
   constexpr int KS = kWarps / MT;   // shares of a staged tile
   constexpr int KW = kKT / KS;      // positions of a share
   constexpr int LDS = lds_for(NT);
@@ -110,9 +114,9 @@ __global__ void __launch_bounds__(kThreads, 2) pk64_kernel(Args a)
   const int mt = warp % MT, ks = warp / MT;
   const int c0 = blockIdx.y * NP;
   const int row0 = (blockIdx.x * MT + mt) * 16 + g;
-  // this part's tiles
+  // this block's tiles
   const int tiles = (K + kKT - 1) / kKT;
-  const int tb = (int)((int64_t)tiles * blockIdx.z / a.nparts), te = (int)((int64_t)tiles * (blockIdx.z + 1) / a.nparts);
+  const int tb = (int)((int64_t)tiles * blockIdx.z / gridDim.z), te = (int)((int64_t)tiles * (blockIdx.z + 1) / gridDim.z);
 
   double3 ox[2], on[2];
 #pragma unroll
@@ -220,124 +224,59 @@ __global__ void __launch_bounds__(kThreads, 2) pk64_kernel(Args a)
     __syncthreads();
   }
 
-  // sum the shares of the tiles in order: share s hands its block to share 0
-  if (KS > 1) {
-    constexpr int LR = NT * 4 * 32 + 0;  // doubles per warp: lane-major accumulators
+  // sum the shares of the tiles in order: share s adds its block to slot mt
+  // of [MT][16][NP] once share s - 1 has
+  double *slot = sm64;
+  constexpr int ROWS = MT * 16;
 #pragma unroll 1
-    for (int s = 1; s < KS; ++s) {
-      if (ks == s) {
-        double *d = sm64 + mt * LR + lane;
+  for (int s = 0; s < KS; ++s) {
+    if (ks == s) {
+      double *d = slot + mt * 16 * NP;
 #pragma unroll
-        for (int j = 0; j < NT; ++j)
+      for (int j = 0; j < NT; ++j)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) d[(j * 4 + q) * 32] = acc[j][q];
-      }
-      __syncthreads();
-      if (ks == 0) {
-        const double *d = sm64 + mt * LR + lane;
-#pragma unroll
-        for (int j = 0; j < NT; ++j)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[j][q] += d[(j * 4 + q) * 32];
-      }
-      __syncthreads();
-    }
-  }
-
-  if (a.nparts > 1) {
-    if (ks == 0) {
-      double *o = a.parts + (size_t)blockIdx.z * M * a.R;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int i = row0 + 8 * h;
-        if (i < M)
-#pragma unroll
-          for (int j = 0; j < NT; ++j)
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const int c = c0 + j * 8 + 2 * t + q;
-              if (c < a.R) o[(size_t)i * a.R + c] = acc[j][2 * h + q];
-            }
-      }
-    }
-    return;
-  }
-  double *red = sm64;  // [MT][NP] curvature partials of the warps
-  if (ks == 0) {
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      double d[2] = {0.0, 0.0};
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int i = row0 + 8 * h;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int c = c0 + j * 8 + 2 * t + q;
-          if (i < M && c < a.R) {
-            const double v = a.coef * acc[j][2 * h + q];
-            a.out[(size_t)i * a.R + c] = v;
-            if (a.part) d[q] += a.pdot[(size_t)i * a.R + c] * v;
-          }
+        for (int q = 0; q < 4; ++q) {
+          double *e = d + (g + 8 * (q >> 1)) * NP + j * 8 + 2 * t + (q & 1);
+          *e = s == 0 ? acc[j][q] : *e + acc[j][q];
         }
-      }
-      if (a.part) {
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-#pragma unroll
-          for (int o = 4; o < 32; o <<= 1) d[q] += __shfl_xor_sync(0xffffffffu, d[q], o);
-          if (g == 0) red[mt * NP + j * 8 + 2 * t + q] = d[q];
-        }
-      }
+    }
+    __syncthreads();
+  }
+  // the cluster's blocks hold their parts of the reduction: each adds and
+  // stores a slice of the outputs
+  namespace cg = cooperative_groups;
+  const int z = gridDim.z;
+  int rank = 0, ra = 0, rb = ROWS;
+  if (z > 1) {
+    cg::cluster_group cl = cg::this_cluster();
+    rank = (int)cl.block_rank();
+    ra = ROWS * rank / z;
+    rb = ROWS * (rank + 1) / z;
+    cl.sync();
+  }
+  __shared__ double red[kThreads];
+  constexpr int RG = kThreads / NP;  // row groups of the store
+  const int c = tid % NP, rg = tid / NP, o0 = blockIdx.x * ROWS;
+  double d = 0.0;
+  if (rg < RG && c0 + c < a.R) {
+    for (int o = ra + rg; o < rb && o0 + o < M; o += RG) {
+      double v = z > 1 ? *cg::this_cluster().map_shared_rank(slot + o * NP + c, 0) : slot[o * NP + c];
+      for (int k = 1; k < z; ++k) v += *cg::this_cluster().map_shared_rank(slot + o * NP + c, k);
+      v *= a.coef;
+      const size_t at = (size_t)(o0 + o) * a.R + c0 + c;
+      a.out[at] = v;
+      if (a.part) d += a.pdot[at] * v;
     }
   }
   if (a.part) {
+    red[tid] = d;
     __syncthreads();
-    for (int c = tid; c < NP; c += kThreads)
-      if (c0 + c < a.R) {
-        double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < MT; ++w) s += red[w * NP + c];
-        a.part[(size_t)blockIdx.x * a.R + c0 + c] = s;
-      }
-  }
-}
-
-// out = coef * the partial blocks in order (M x R each), with the curvature
-// partials of kSumRows rows per block
-constexpr int kSumRows = 64;
-static __global__ void __launch_bounds__(256) pk64_sum_kernel(int M, int R, int nparts, const double *__restrict__ parts,
-                                                              double coef, double *__restrict__ out,
-                                                              const double *__restrict__ pdot, double *__restrict__ part,
-                                                              const int32_t *__restrict__ done)
-{
-  if (done && *done) return;
-  const int i0 = blockIdx.x * kSumRows, i1 = min(M, i0 + kSumRows);
-  const size_t stride = (size_t)M * R;
-  __shared__ double red[8][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int cb = 0; cb < R; cb += 32) {
-    const int c = cb + lane;
-    double d = 0.0;
-    if (c < R)
-      for (int i = i0 + warp; i < i1; i += 8) {
-        const size_t o = (size_t)i * R + c;
-        double s = parts[o];
-        for (int z = 1; z < nparts; ++z) s += parts[z * stride + o];
-        s *= coef;
-        out[o] = s;
-        if (part) d += pdot[o] * s;
-      }
-    if (part) {
-      red[warp][lane] = d;
-      __syncthreads();
-      if (warp == 0 && c < R) {
-#pragma unroll
-        for (int w = 1; w < 8; ++w) d += red[w][lane];
-        part[(size_t)blockIdx.x * R + c] = d;
-      }
-      __syncthreads();
+    if (rg == 0 && c0 + c < a.R) {
+      for (int k = 1; k < RG; ++k) d += red[k * NP + c];
+      a.part[((size_t)blockIdx.x * z + rank) * a.R + c0 + c] = d;
     }
   }
+  if (z > 1) cg::this_cluster().sync();  // no block leaves while others read its sums
 }
 
 }  // namespace p64

@@ -8,9 +8,7 @@
 namespace mbc {
 
 // most rows of curvature partials a columns product of n sources writes
-inline int p64_part_rows(int n) { return (n + 15) / 16; }
-// size the buffer of split products of R columns (before a stream capture)
-mbc_status p64_reserve(const Solver &S, int R);
+inline int p64_part_rows(int n) { return (n + 63) / 64 * 8; }
 // w (nf x R) = K v
 void p64_launch_rows(const Solver &S, int R, const double *v, double *w, const int32_t *done, cudaStream_t st);
 // t (n x R) = K^T w, optionally with the partials of p . t; returns their rows

@@ -200,6 +200,11 @@ __device__ __forceinline__ uint64_t digit_bytes(double v, int a)
 // slab by slab (rows [rt0, rt0 + gridDim.y) tiles) for every matvec.
 constexpr int kModeExps = 1;
 constexpr int kModeDigits = 2;
+// two doubles of padding per 16: the eight 16-position groups of a warp read
+// different banks
+constexpr int kChunkPad = kChunk + kChunk / 8;
+__host__ __device__ constexpr int pad16(int k) { return k + ((k >> 4) << 1); }
+__host__ __device__ constexpr int digits_smem(int dir) { return (dir == 0 ? 3 : 6) * kChunkPad * (int)sizeof(double); }
 
 // ---------------------------------------------------------------------------
 // A digit planes of G for one direction.  Grid (chunks, row tiles of the
@@ -208,8 +213,9 @@ constexpr int kModeDigits = 2;
 // with the swizzled tile image; aexp[(rt * nchunks + c) * kM + row].  Rows or
 // K positions past the ends get digit 0.  A non-finite G (coincident point
 // and source) sets *err = 3 and counts as 0.
-// Shared memory: kChunk float4 (DIR 0: sources) or 2 kChunk (DIR 1: points,
-// normals).
+// Shared memory: the chunk's points as doubles, digits_smem(DIR): converting
+// them in every evaluation (nine conversions) costs more than its 16 FP64
+// instructions.
 template <int DIR>
 __global__ void __launch_bounds__(256) oz_digits_kernel(const float4 *__restrict__ xr,
                                                         const float4 *__restrict__ nr,
@@ -220,7 +226,7 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const float4 *__restrict
                                                         int32_t *__restrict__ err)
 {
   if (done && *done) return;  // a slab rebuild after the PCG stopped
-  extern __shared__ float4 sco[];
+  extern __shared__ double sco[];  // [3 or 6][kChunkPad]: sources, or points and normals
   const int M = DIR == 0 ? nf : n;
   const int K = DIR == 0 ? n : nf;
   const int c = blockIdx.x, rt = rt0 + (int)blockIdx.y, rt_local = (int)blockIdx.y;
@@ -232,35 +238,38 @@ __global__ void __launch_bounds__(256) oz_digits_kernel(const float4 *__restrict
   const int kcount = min(kChunk, K - kbase);
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int t = threadIdx.x; t < kChunk; t += blockDim.x) {
-    if (DIR == 0) {
-      sco[t] = t < kcount ? ys[kbase + t] : zero;
-    } else {
-      sco[t] = t < kcount ? xr[kbase + t] : zero;
-      sco[kChunk + t] = t < kcount ? nr[kbase + t] : zero;
+    const float4 p = t < kcount ? (DIR == 0 ? ys[kbase + t] : xr[kbase + t]) : zero;
+    double *d = sco + pad16(t);
+    d[0] = p.x;
+    d[kChunkPad] = p.y;
+    d[2 * kChunkPad] = p.z;
+    if (DIR == 1) {
+      const float4 q = t < kcount ? nr[kbase + t] : zero;
+      d[3 * kChunkPad] = q.x;
+      d[4 * kChunkPad] = q.y;
+      d[5 * kChunkPad] = q.z;
     }
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane >> 3, c16 = lane & 7;  // row of the warp's four, 16-byte group of the row
-  float4 own[4], own_n[4];
+  double3 own[4], own_n[4];
   bool valid[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const int gm = rt * kM + 32 * u + 4 * warp + sub;
     valid[u] = gm < M;
-    own[u] = own_n[u] = zero;
-    if (valid[u]) {
-      if (DIR == 0) {
-        own[u] = xr[gm];
-        own_n[u] = nr[gm];
-      } else {
-        own[u] = ys[gm];
-      }
-    }
+    const float4 p = valid[u] ? (DIR == 0 ? xr[gm] : ys[gm]) : zero;
+    const float4 q = DIR == 0 && valid[u] ? nr[gm] : zero;
+    own[u] = make_double3(p.x, p.y, p.z);
+    own_n[u] = make_double3(q.x, q.y, q.z);
   }
   auto eval = [&](int u, int k) -> double {
-    return DIR == 0 ? PointKernel<double>::eval(own[u], own_n[u], sco[k])
-                    : PointKernel<double>::eval(sco[k], sco[kChunk + k], own[u]);
+    const double *d = sco + pad16(k);
+    const double3 p = make_double3(d[0], d[kChunkPad], d[2 * kChunkPad]);
+    return DIR == 0 ? PointKernel<double>::eval(own[u], own_n[u], p)
+                    : PointKernel<double>::eval(
+                          p, make_double3(d[3 * kChunkPad], d[4 * kChunkPad], d[5 * kChunkPad]), own[u]);
   };
   // pass 1: the largest |G| of each row over the chunk
   double mx[4] = {0.0, 0.0, 0.0, 0.0};

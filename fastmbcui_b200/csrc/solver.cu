@@ -221,8 +221,8 @@ int launch_cols(const Solver &S, int R, const T *w, T *t, const T *pdot, double 
 }
 
 // upper bound on the blocks of any columns-direction launch (the per-block
-// curvature partials): FP64 tiles of 16 sources or more, SIMT 64, tensor cores
-// 128, dense 64 in clusters of up to 8
+// curvature partials): FP64 and dense tiles of 64 sources in clusters of up
+// to 8, SIMT 64, tensor cores 128
 int cols_blocks(const Solver &S) { return std::max(p64_part_rows(S.n), dense_part_rows(S.n)); }
 
 template void launch_rows<float>(const Solver &, int, const float *, float *, const int32_t *, cudaStream_t);
@@ -685,7 +685,6 @@ static mbc_status pcg_buffers_in(Solver &S, int R, PcgWork<T> &w, DevMem &m, Dev
   w.sc.stall = ii + 2 * R + 4;
   w.sc.drop2 = 0.0;
   w.sc.stall_check = 1;
-  if (sizeof(T) == 8) p64_reserve(S, R);  // without the buffer the products run unsplit
   return MBC_OK;
 }
 

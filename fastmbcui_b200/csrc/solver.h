@@ -47,7 +47,6 @@ struct Solver {
   DevMem m_z4;  // mesh operator: third vertex of every face (x4, n4 hold the first two)
   DevMem m_err;           // set by a tensor-core kernel (1: a bounded wait expired)
   uint32_t wait_limit = 0;  // polls before a tensor-core kernel's partner wait gives up (0: the default)
-  mutable DevMem m_p64;   // partial blocks of split FP64 products (matvec64.cu)
   mutable std::bitset<128> p64_smem;  // matvec64.cu kernels whose shared memory is allowed (this solver's device)
   mutable std::bitset<32> dense_smem;  // ... and the dense.cu kernels
   mutable DevMem m_bimg;  // packed TF32 hi/lo image of the tensor-core B operand
