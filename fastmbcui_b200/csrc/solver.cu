@@ -553,6 +553,14 @@ mbc_status Solver::factor(cudaStream_t st)
       return fail(MBC_NONSPD_PIVOT, std::to_string(nbad) + " supernode(s) not positive definite");
     }
   }
+  // L's values once more in row order: the preconditioner's z = L u walks rows
+  MBC_TRY(lrow.reserve(std::max<size_t>(l_n * esz, 16)));
+  if (precision == MBC_F64)
+    row_values_kernel<double><<<cdiv(l_n, 256), 256, 0, st>>>((int64_t)l_n, d_rmap(), (const double *)lval.ptr, (double *)lrow.ptr);
+  else
+    row_values_kernel<float><<<cdiv(l_n, 256), 256, 0, st>>>((int64_t)l_n, d_rmap(), (const float *)lval.ptr, (float *)lrow.ptr);
+  MBC_CKL();
+  MBC_CK(cudaStreamSynchronize(st));
   factored = true;
   return MBC_OK;
 }
@@ -628,12 +636,57 @@ Layout2D layout2d(int n, int R)
   const int by = 256 / bx;
   Layout2D L;
   L.block = dim3(bx, by);
-  L.grid = dim3(cdiv(n, by), cdiv(R, bx));
+  // about eight blocks per SM, striding over the rows: the partials stay few
+  const unsigned gy = cdiv(R, bx);
+  L.grid = dim3(std::min<unsigned>(cdiv(n, by), std::max(8u * 148u / gy, 1u)), gy);
   L.smem = sizeof(double) * 256;
   return L;
 }
 
 }  // namespace
+
+// Sums of nblk partials of R columns and their step (reduce_kernel).
+static void launch_reduce(cudaStream_t st, int nblk, int R, const double *part, int32_t mode, const PcgScalars &sc,
+                          double *out)
+{
+  reduce_kernel<<<cdiv(R, 8), 256, 0, st>>>(nblk, R, part, mode, sc, out);
+}
+
+// Whether the kernel that writes nblk partials of R columns sums them itself
+// (its last block; ~4 us less per reduction at R = 6, slower from a few
+// thousand sums of 32 on, which eight warps walk alone)
+static bool reduce_in_place(int nblk, int R) { return (int64_t)cdiv(nblk, 32) * R <= 256; }
+
+// The two halves of the preconditioner, z = L (L^T r); with `part` the second
+// forms the partials of r . z and, for mode RED_BETA, their reduction.
+// Warps per row: as many as keep ~16 warps per SM busy in small scenes.
+struct PrecondShape {
+  dim3 grid;
+  int cx, wpr;
+};
+static PrecondShape precond_shape(int n, int R)
+{
+  PrecondShape s{};
+  s.cx = 1;
+  while (s.cx < R && s.cx < 32) s.cx <<= 1;
+  const unsigned gy = cdiv(R, s.cx);
+  s.wpr = 1;
+  while (s.wpr < 8 && (int64_t)n * gy * s.wpr < 16 * 148) s.wpr <<= 1;
+  s.grid = dim3(std::min<unsigned>(cdiv(n, 8 / s.wpr), std::max(8u * 148u / gy, 1u)), gy);
+  return s;
+}
+template <typename T, typename LT>
+static int launch_precond(const Solver &S, int R, const LT *lval, const T *r, T *u, T *z, double *part, int32_t mode,
+                          const PcgScalars &sc, const int32_t *done, cudaStream_t st)
+{
+  const PrecondShape s = precond_shape(S.n, R);
+  precond_kernel<T, LT><<<s.grid, 256, 0, st>>>(S.n, R, s.cx, s.wpr, S.d_lptr(), S.d_lind(), lval, r, u, nullptr,
+                                               nullptr, RED_NONE, sc, done);
+  precond_kernel<T, LT><<<s.grid, 256, 0, st>>>(S.n, R, s.cx, s.wpr, S.d_rptr(), S.d_rcol(), (const LT *)S.lrow.ptr, u, z, r,
+                                               part, mode, sc, done);
+  S.launches += 2;
+  return (int)s.grid.x;
+}
 
 // Work buffers for one precision.  X64 is the FP64 solution accumulator of
 // the residual-replacement mode.
@@ -663,7 +716,7 @@ static mbc_status pcg_buffers_in(Solver &S, int R, PcgWork<T> &w, DevMem &m, Dev
   w.U = (T *)(b + 4 * vb);
   w.Tt = (T *)(b + 5 * vb);
   w.W = (T *)(b + 6 * vb);
-  const int nblk = std::max<int>(std::max<int>(cols_blocks(S), layout2d(S.n, R).grid.x), 1);
+  const int nblk = std::max({cols_blocks(S), (int)layout2d(S.n, R).grid.x, (int)precond_shape(S.n, R).grid.x, 1});
   w.part_stride = nblk;
   MBC_TRY(part.reserve(sizeof(double) * (size_t)nblk * R));
   w.part = (double *)part.ptr;
@@ -682,6 +735,7 @@ static mbc_status pcg_buffers_in(Solver &S, int R, PcgWork<T> &w, DevMem &m, Dev
   w.sc.iters = ii + R;
   w.sc.done = ii + 2 * R;
   w.sc.want = ii + 2 * R + 1;
+  w.sc.tick = ii + 2 * R + 2;
   w.sc.stall = ii + 2 * R + 4;
   w.sc.drop2 = 0.0;
   w.sc.stall_check = 1;
@@ -695,12 +749,13 @@ static mbc_status pcg_buffers(Solver &S, int R, PcgWork<T> &w)
 }
 
 __global__ void set_status_kernel(int R, int32_t *status, int32_t *iters, int32_t *done,
-                                  int32_t *want, double *rz, const int32_t *mask)
+                                  int32_t *want, int32_t *tick, double *rz, const int32_t *mask)
 {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c == 0) {
     *done = 0;
     *want = 0;
+    tick[0] = tick[1] = 0;
   }
   if (c >= R) return;
   status[c] = (mask == nullptr || mask[c]) ? COL_ACTIVE : COL_OK;
@@ -750,10 +805,10 @@ static mbc_status run_pcg(Solver &S, int R, PcgWork<T> &w, XT *x, const LT *lval
   w.sc.maxit = maxit;
   w.sc.tol2 = tol * tol;
   set_status_kernel<<<cdiv(R, 256), 256, 0, st>>>(R, w.sc.status, w.sc.iters, w.sc.done, w.sc.want,
-                                                   w.sc.rz, d_mask);
+                                                   w.sc.tick, w.sc.rz, d_mask);
   // |b|^2 and the stopping thresholds
   dot_partial_kernel<T><<<L.grid, L.block, L.smem, st>>>(S.n, R, w.Rv, w.Rv, w.part);
-  reduce_kernel<<<1, 1024, 0, st>>>(nblk2, R, w.part, RED_INIT_B, w.sc, nullptr);
+  launch_reduce(st, nblk2, R, w.part, RED_INIT_B, w.sc, nullptr);
   if (d_b2ref) set_thresholds_kernel<<<cdiv(R, 256), 256, 0, st>>>(R, w.sc.tol2, d_b2ref, w.sc);
   MBC_CK(cudaMemsetAsync(w.Pv, 0, sizeof(T) * (size_t)S.n * R, st));
   MBC_CKL();
@@ -803,27 +858,33 @@ static mbc_status run_pcg(Solver &S, int R, PcgWork<T> &w, XT *x, const LT *lval
     if (use_graph && !graph.exec) MBC_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
     for (int k = 0; k < kmax && !(use_graph && graph.exec && graph_launches > 0); ++k) {
       if (precond) {
-        precond_lt_kernel<T, LT><<<cL.grid, cL.block, 0, st>>>(S.n, cR, S.d_lptr(), S.d_lind(), lval,
-                                                                cw->Rv, cw->U, cw->sc.done);
-        precond_l_kernel<T, LT><<<cL.grid, cL.block, cL.smem, st>>>(S.n, cR, S.d_rptr(), S.d_rcol(),
-                                                                   S.d_rmap(), lval, cw->U, cw->Z, cw->Rv,
-                                                                   cw->part, cw->sc.done);
+        const int nbp = (int)precond_shape(S.n, cR).grid.x;
+        const bool own = reduce_in_place(nbp, cR);
+        launch_precond<T, LT>(S, cR, lval, cw->Rv, cw->U, cw->Z, cw->part, own ? RED_BETA : RED_NONE, cw->sc,
+                              cw->sc.done, st);
+        if (!own) {
+          launch_reduce(st, nbp, cR, cw->part, RED_BETA, cw->sc, nullptr);
+          ++S.launches;
+        }
       } else {
         MBC_CK(cudaMemcpyAsync(cw->Z, cw->Rv, sizeof(T) * (size_t)S.n * cR, cudaMemcpyDeviceToDevice, st));
         dot_partial_kernel<T><<<cL.grid, cL.block, cL.smem, st>>>(S.n, cR, cw->Rv, cw->Z, cw->part);
+        launch_reduce(st, cnblk2, cR, cw->part, RED_BETA, cw->sc, nullptr);
+        S.launches += 2;
       }
-      reduce_kernel<<<1, 1024, 0, st>>>(cnblk2, cR, cw->part, RED_BETA, cw->sc, nullptr);
       update_p_kernel<T><<<cL.grid, cL.block, 0, st>>>(S.n, cR, cw->sc.beta, cw->sc.status, cw->Z, cw->Pv,
                                                         cw->sc.done);
+      const bool in_place = reduce_in_place(cnblk2, cR);
       if (S.profile) MBC_CK(cudaEventRecord(S.events[2 * k], st));
       launch_rows<T>(S, cR, cw->Pv, cw->W, cw->sc.done, st);
       const int nb = launch_cols<T>(S, cR, cw->W, cw->Tt, cw->Pv, cw->part, cw->sc.done, st);
       if (S.profile) MBC_CK(cudaEventRecord(S.events[2 * k + 1], st));
-      reduce_kernel<<<1, 1024, 0, st>>>(nb, cR, cw->part, RED_ALPHA, cw->sc, nullptr);
+      launch_reduce(st, nb, cR, cw->part, RED_ALPHA, cw->sc, nullptr);
       update_xr_kernel<T, XT><<<cL.grid, cL.block, cL.smem, st>>>(S.n, cR, cw->sc.alpha, cw->Pv, cw->Tt, cx,
-                                                                 cw->Rv, cw->part, cw->sc.done);
-      reduce_kernel<<<1, 1024, 0, st>>>(cnblk2, cR, cw->part, RED_CHECK, cw->sc, nullptr);
-      S.launches += precond ? 7 : 6;  // the matvec pair counts itself
+                                                                 cw->Rv, cw->part, in_place ? RED_CHECK : RED_NONE, cw->sc,
+                                                                 cw->sc.done);
+      if (!in_place) launch_reduce(st, cnblk2, cR, cw->part, RED_CHECK, cw->sc, nullptr);
+      S.launches += in_place ? 3 : 4;  // the preconditioner and the matvec pair count themselves
     }
     if (use_graph && !graph.exec) {
       cudaGraph_t g = nullptr;
@@ -973,10 +1034,10 @@ static mbc_status run_block_pcg(Solver &S, int R, PcgWork<double> &w, const LT *
   const Layout2D L0 = layout2d(n, R);
   w.sc.maxit = maxit;
   w.sc.tol2 = tol * tol;
-  set_status_kernel<<<cdiv(R, 256), 256, 0, st>>>(R, w.sc.status, w.sc.iters, w.sc.done, w.sc.want, w.sc.rz,
-                                                   nullptr);
+  set_status_kernel<<<cdiv(R, 256), 256, 0, st>>>(R, w.sc.status, w.sc.iters, w.sc.done, w.sc.want,
+                                                   w.sc.tick, w.sc.rz, nullptr);
   dot_partial_kernel<double><<<L0.grid, L0.block, L0.smem, st>>>(n, R, w.Rv, w.Rv, w.part);
-  reduce_kernel<<<1, 1024, 0, st>>>((int)L0.grid.x, R, w.part, RED_INIT_B, w.sc, nullptr);
+  launch_reduce(st, (int)L0.grid.x, R, w.part, RED_INIT_B, w.sc, nullptr);
   if (d_b2ref) set_thresholds_kernel<<<cdiv(R, 256), 256, 0, st>>>(R, w.sc.tol2, d_b2ref, w.sc);
   S.launches += d_b2ref ? 4 : 3;
   MBC_CKL();
@@ -1009,11 +1070,7 @@ static mbc_status run_block_pcg(Solver &S, int R, PcgWork<double> &w, const LT *
     ++S.launches;
   };
   auto precond = [&](int a, const double *Rm, double *Zm) {
-    const Layout2D La = layout2d(n, a);
-    precond_lt_kernel<double, LT><<<La.grid, La.block, 0, st>>>(n, a, S.d_lptr(), S.d_lind(), lval, Rm, U, nullptr);
-    precond_l_kernel<double, LT><<<La.grid, La.block, La.smem, st>>>(n, a, S.d_rptr(), S.d_rcol(), S.d_rmap(), lval,
-                                                                      U, Zm, Rm, w.part, nullptr);
-    S.launches += 2;
+    launch_precond<double, LT>(S, a, lval, Rm, U, Zm, nullptr, RED_NONE, PcgScalars{}, nullptr, st);
   };
   // the small factorizations keep their matrix's lower triangle in shared
   // memory (packed) when it fits; the column-parallel solves add one column
@@ -1082,7 +1139,7 @@ static mbc_status run_block_pcg(Solver &S, int R, PcgWork<double> &w, const LT *
     const Layout2D La = layout2d(n, a);
     dot_partial_kernel<double><<<La.grid, La.block, La.smem, st>>>(n, a, Ra[cur], Ra[cur], w.part);
     PcgScalars none{};
-    reduce_kernel<<<1, 1024, 0, st>>>((int)La.grid.x, a, w.part, RED_STORE, none, rr);
+    launch_reduce(st, (int)La.grid.x, a, w.part, RED_STORE, none, rr);
     block_check_kernel<<<cdiv(a, 256), 256, 0, st>>>(a, d_act, rr, w.sc);
     S.launches += 6;
     MBC_CKL();
@@ -1179,7 +1236,7 @@ static mbc_status col_norms2(Solver &S, int R, const T *A, std::vector<double> &
   double *res = part + (size_t)L.grid.x * R;
   dot_partial_kernel<T><<<L.grid, L.block, L.smem, st>>>(S.n, R, A, A, part);
   PcgScalars sc{};
-  reduce_kernel<<<1, 1024, 0, st>>>((int)L.grid.x, R, part, RED_STORE, sc, res);
+  launch_reduce(st, (int)L.grid.x, R, part, RED_STORE, sc, res);
   S.launches += 2;
   MBC_CKL();
   out.resize(R);
@@ -1197,7 +1254,7 @@ static mbc_status col_norms2_dev(Solver &S, int R, const T *A, double *out, cuda
   double *part = (double *)S.nrm.ptr;
   dot_partial_kernel<T><<<L.grid, L.block, L.smem, st>>>(S.n, R, A, A, part);
   PcgScalars sc{};
-  reduce_kernel<<<1, 1024, 0, st>>>((int)L.grid.x, R, part, RED_STORE, sc, out);
+  launch_reduce(st, (int)L.grid.x, R, part, RED_STORE, sc, out);
   S.launches += 2;
   MBC_CKL();
   return MBC_OK;
@@ -1573,7 +1630,7 @@ mbc_status Solver::solve_mixed(int R, const void *rhs, int32_t rhs_dt, void *X, 
   std::function<mbc_status()> replace = [&]() -> mbc_status {
     MBC_TRY(true_residual_into_r());
     dot_partial_kernel<double><<<L.grid, L.block, L.smem, st>>>(n, R, Rd, Rd, w.part);
-    reduce_kernel<<<1, 1024, 0, st>>>((int)L.grid.x, R, w.part, RED_REPLACE, w.sc, nullptr);
+    launch_reduce(st, (int)L.grid.x, R, w.part, RED_REPLACE, w.sc, nullptr);
     launches += 2;
     MBC_CKL();
     return MBC_OK;

@@ -60,7 +60,7 @@ struct Solver {
   DevMem m_oz_q[2], m_oz_ys, m_oz_xr, m_oz_nr;
   DevMem m_oz_chk;  // the self-check's vectors
   // factor
-  DevMem theta, theta64, lval, bad, fscratch;
+  DevMem theta, theta64, lval, lrow, bad, fscratch;  // lrow: lval in row order
   // PCG workspaces
   DevMem work32, work64, part, scal, fbuf32, fbuf64, res64, mask, colbuf, tmp, b2ref, nrm, polish_idx;
   DevMem blk;  // block PCG: compact column blocks, search blocks, small matrices
