@@ -18,6 +18,16 @@
 
 namespace mbc {
 
+// The hardware estimate without rsqrtf's scaling of denormal arguments (four
+// instructions of sixteen in an evaluation): for those the kernel value
+// itself is beyond FP32's range.
+__device__ __forceinline__ float rsqrt_ftz(float a)
+{
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+
 template <typename T>
 struct PointKernel;
 
@@ -27,7 +37,7 @@ struct PointKernel<float> {
   {
     const float dx = x.x - y.x, dy = x.y - y.y, dz = x.z - y.z;
     const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-    const float ir = rsqrtf(r2);
+    const float ir = rsqrt_ftz(r2);
     const float rn = fmaf(dz, nx.z, fmaf(dy, nx.y, dx * nx.x));
     return rn * (ir * ir * ir);
   }

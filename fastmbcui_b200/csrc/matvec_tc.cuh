@@ -21,16 +21,18 @@
 //     128-byte swizzle), so a stage is one contiguous bulk copy.
 //   pk_tc_kernel: one CTA owns 128 outputs (accumulator of 128 lanes x np
 //     columns in tensor memory; np = R padded to 16) and walks the k-steps of
-//     32 through two shared-memory rings: 2 stages of A (the G tile, hi and
-//     lo) and 3 stages (2 when np > 192) of B image + coordinates, so the bulk
-//     copy of a step is issued two MMA steps before it is needed:
+//     32 through two shared-memory rings: 4 stages of A (the G tile, hi and
+//     lo; 2 when np > 112) and 2 to 5 of B image + coordinates, so the bulk
+//     copy of a step is issued well before it is needed:
 //       loader warp  -- waits "bempty", bulk-copies the stage's coordinates
 //                       and B image (cp.async.bulk, completion on "bfull");
-//       16 producer warps -- wait "bfull" and "aempty", evaluate the 128 x 32
-//                       tile of G in FP32 from the staged coordinates, split,
-//                       store A hi / lo swizzled, fence to the async proxy,
-//                       arrive on "afull";
-//       MMA warp     -- waits "afull" and "bfull" (and, at a chunk start,
+//       scheduler warp -- waits "bfull" and "aempty" of a step and releases
+//                       the producer group whose turn it is ("go");
+//       16 producer warps in two groups, a k-step each in turn -- evaluate the
+//                       128 x 32 tile of G in FP32 from the staged
+//                       coordinates, split, store A hi / lo swizzled, fence to
+//                       the async proxy, meet the MMA warp ("A ready");
+//       MMA warp     -- waits "A ready" and "bfull" (and, at a chunk start,
 //                       "chunk_free"), issues 4 x 3 tcgen05.mma (kind::tf32,
 //                       K = 8), commits to "aempty" and "bempty" and, at a
 //                       chunk end, "chunk_full";
@@ -39,6 +41,13 @@
 //                       arrive "chunk_free"; after the last chunk they scale
 //                       by coef and store, and in the columns direction form
 //                       the PCG curvature partials p.t per CTA.
+// A launch with few tiles, or a short last wave, cuts the k-steps over grid.y
+// into parts that sum_parts_kernel adds in order.
+// What bounds it: shared memory, ~1700 of the ~2000 cycles of a k-step at 96
+// columns (MMA operand reads 660, producer stores and coordinate loads 770 to
+// 1100, bulk copies 200); the producers issue for 990.  Measured (B200): K and
+// K^T of 64000 x 64000, 96 columns 20.2 -> 14.1 ms against one producer group,
+// two A stages, cvt.rna.tf32 and no parts; 9600 outputs, 36 columns 0.38 -> 0.2 ms.
 // Every mbarrier wait is bounded: on expiry the kernel records the failure in
 // *err, stops waiting, releases the waiters it feeds, waits (bounded) for its
 // own copies, frees its tensor memory and returns.
@@ -54,10 +63,12 @@ namespace tc {
 
 constexpr int kM = 128;     // MMA M (outputs per CTA)
 constexpr int kK = 32;      // k-step: one 128-byte swizzle row of TF32
-constexpr int kAStages = 2;     // ring of produced A (G) tiles
-constexpr int kMaxBStages = 3;  // ring of bulk-copied B image + coordinates
+constexpr int kMaxAStages = 4;  // ring of produced A (G) tiles
+constexpr int kMaxBStages = 5;  // ring of bulk-copied B image + coordinates
 constexpr int kChunk = 32;  // k-steps accumulated in tensor memory before a fold
 constexpr int kProducerWarps = 16;
+constexpr int kGroups = 2;      // producer groups, one k-step each in turn
+constexpr int kGroupWarps = kProducerWarps / kGroups;
 constexpr int kLoaderWarp = kProducerWarps;
 constexpr int kMmaWarp = kProducerWarps + 1;
 constexpr int kAccWarp0 = kProducerWarps + 2;  // 4 accumulator warps
@@ -65,17 +76,16 @@ constexpr int kSchedWarp = kProducerWarps + 6;
 constexpr int kThreads = (kProducerWarps + 7) * 32;
 // named barriers (0 is __syncthreads).  Every participant uses bar.sync, so
 // no role can run more than one step ahead of a partner.
-constexpr int kBarGo = 1;      // producers + scheduler warp, once per k-step
-constexpr int kBarAReady = 2;  // producers + MMA warp, once per k-step
-constexpr int kBarAcc = 3;     // the 4 accumulator warps, once per chunk
-constexpr int kGoCount = (kProducerWarps + 1) * 32;
-constexpr int kKPerProducer = kK / (kProducerWarps / 4);  // k values per row per k-step
+constexpr int kBarGo = 1;                    // + group: its producers and the scheduler warp, once per k-step
+constexpr int kBarAReady = kBarGo + kGroups; // + group: its producers and the MMA warp, once per k-step
+constexpr int kBarAcc = kBarAReady + kGroups;  // the 4 accumulator warps, once per chunk
+constexpr int kGoCount = (kGroupWarps + 1) * 32;
+constexpr int kKPerProducer = kK / (kGroupWarps / 4);  // k values per row per k-step
 constexpr uint32_t kWaitLimit = 1u << 22;  // polls of a bounded wait
 constexpr int kSmemLimit = 232448;        // opt-in dynamic shared memory per CTA (227 KB)
 constexpr int kTail = 256 + 8192;         // barriers, then the accumulator warps' partials
 
 constexpr int kTileA = kM * kK * 4;  // one A operand tile: 16 KB
-constexpr int kABytes = kAStages * 2 * kTileA;
 
 __host__ __device__ constexpr int tile_b_bytes(int np) { return np * kK * 4; }
 __host__ __device__ constexpr int coord_bytes(int dir) { return dir == 0 ? kK * 16 : kK * 32; }
@@ -84,14 +94,23 @@ __host__ __device__ constexpr int bstage_bytes(int np, int dir)
 {
   return (2 * tile_b_bytes(np) + coord_bytes(dir) + 1023) / 1024 * 1024;
 }
+// A stages: four where three B stages still fit beside them (np <= 112), so
+// that both producer groups work while the MMAs of a step run; else two
+__host__ __device__ constexpr int a_stages(int np, int dir)
+{
+  return kMaxAStages * 2 * kTileA + 3 * bstage_bytes(np, dir) + kTail <= kSmemLimit ? kMaxAStages : 2;
+}
+__host__ __device__ constexpr int a_bytes(int np, int dir) { return a_stages(np, dir) * 2 * kTileA; }
 __host__ __device__ constexpr int b_stages(int np, int dir)
 {
-  return kABytes + kMaxBStages * bstage_bytes(np, dir) + kTail <= kSmemLimit ? kMaxBStages : 2;
+  int n = kMaxBStages;
+  while (n > 2 && a_bytes(np, dir) + n * bstage_bytes(np, dir) + kTail > kSmemLimit) --n;
+  return n;
 }
 // [A ring | B ring | tail]; the dynamic shared window starts 1024-aligned
 __host__ __device__ constexpr int smem_bytes(int np, int dir)
 {
-  return kABytes + b_stages(np, dir) * bstage_bytes(np, dir) + kTail;
+  return a_bytes(np, dir) + b_stages(np, dir) * bstage_bytes(np, dir) + kTail;
 }
 
 __host__ __device__ constexpr int tmem_cols_for(int np)
@@ -112,12 +131,11 @@ __host__ __device__ __forceinline__ uint32_t sw128(int row, int k)
                     ((k & 3) << 2));
 }
 
-__device__ __forceinline__ uint32_t tf32_rna(float v)
-{
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
-  return r;
-}
+// nearest TF32 value, ties away from zero, in integer arithmetic: half a unit
+// is added to the magnitude and the 13 low bits dropped.  (cvt.rna.tf32 does
+// the same at a sixteenth of the rate; two per kernel value were a fifth of
+// the producers' time.)
+__device__ __forceinline__ uint32_t tf32_rna(float v) { return (__float_as_uint(v) + 0x1000u) & 0xffffe000u; }
 
 __device__ __forceinline__ void split_tf32(float v, uint32_t &hi, uint32_t &lo)
 {
@@ -297,6 +315,7 @@ struct TcArgs {
   const float *pdot;      // columns: p (n x R) for the curvature partials, or NULL
   double *part;           // columns: per-CTA partials (gridDim.x x R)
   const int32_t *done;    // PCG all-stopped flag (may be NULL)
+  float *parts;           // gridDim.y > 1: [part][M][R] sums of the parts of the reduction, without coef
   int32_t *err;           // 1: a bounded wait expired; 2: shared memory misaligned
   // polls after which a wait for a partner gives up (0: kWaitLimit); the
   // waits that drain the CTA's own copies and MMAs always use kWaitLimit
@@ -312,16 +331,15 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
     if (threadIdx.x == 0) atomicExch(a.err, 2);
     return;
   }
-  const int nbs = b_stages(a.np, DIR);
+  const int nas = a_stages(a.np, DIR), nbs = b_stages(a.np, DIR);
   const int bst = bstage_bytes(a.np, DIR);
   const int btile = tile_b_bytes(a.np);
-  unsigned char *bring = smem + kABytes;
+  unsigned char *bring = smem + a_bytes(a.np, DIR);
   unsigned char *tail = bring + nbs * bst;
   uint64_t *bfull = reinterpret_cast<uint64_t *>(tail);  // B stage landed
   uint64_t *bempty = bfull + kMaxBStages;                 // B stage read by its MMAs
-  uint64_t *afull = bempty + kMaxBStages;                 // A stage written by the producers
-  uint64_t *aempty = afull + kAStages;                    // A stage read by its MMAs
-  uint64_t *chunk_full = aempty + kAStages;
+  uint64_t *aempty = bempty + kMaxBStages;                // A stage read by its MMAs
+  uint64_t *chunk_full = aempty + kMaxAStages;
   uint64_t *chunk_free = chunk_full + 1;
   uint64_t *mma_done = chunk_free + 1;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mma_done + 1);
@@ -333,7 +351,10 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
   const int M_total = DIR == 0 ? a.nf : a.n;
   const int K_total = DIR == 0 ? a.n : a.nf;
   const int m0 = blockIdx.x * kM;
-  const int nks = (K_total + kK - 1) / kK;
+  // this CTA's part of the k-steps: the loops run over ks - ks0
+  const int steps = (K_total + kK - 1) / kK;
+  const int ks0 = (int)((int64_t)steps * blockIdx.y / gridDim.y);
+  const int nks = (int)((int64_t)steps * (blockIdx.y + 1) / gridDim.y) - ks0;
   const int nchunks = (nks + kChunk - 1) / kChunk;
   const int tcols = 2 * a.tmem_cols;  // [chunk accumulator | running sum]
   const uint32_t WL = a.wait_limit ? a.wait_limit : kWaitLimit;
@@ -343,10 +364,7 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
       mbar_init(&bfull[s], 1);
       mbar_init(&bempty[s], 1);
     }
-    for (int s = 0; s < kAStages; ++s) {
-      mbar_init(&afull[s], kProducerWarps);
-      mbar_init(&aempty[s], 1);
-    }
+    for (int s = 0; s < kMaxAStages; ++s) mbar_init(&aempty[s], 1);
     mbar_init(chunk_full, 1);
     mbar_init(chunk_free, 4);
     mbar_init(mma_done, 1);
@@ -374,9 +392,10 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
   volatile int *vfail = s_fail;
   if (warp < kProducerWarps) {
     // ---------------- producers: the G tile ----------------
-    // row 32*(warp%4) + lane, kKPerProducer values of each k-step
+    // row 32*(warp%4) + lane, kKPerProducer values of every kGroups-th k-step
     const int row = (warp & 3) * 32 + lane;
-    const int kbeg = (warp >> 2) * kKPerProducer;
+    const int group = warp / kGroupWarps;
+    const int kbeg = ((warp % kGroupWarps) >> 2) * kKPerProducer;
     const int gm = m0 + row;
     float4 own = make_float4(0.f, 0.f, 0.f, 0.f), own_n = own;
     if (gm < M_total) {
@@ -387,24 +406,23 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
         own = a.ys[gm];
       }
     }
-    for (int ks = 0; ks < nks; ++ks) {
-      const int sa = ks % kAStages, sb = ks % nbs;
-      asm volatile("bar.sync %0, %1;" ::"n"(kBarGo), "n"(kGoCount) : "memory");
+    for (int ks = group; ks < nks; ks += kGroups) {
+      const int sa = ks % nas, sb = ks % nbs;
+      asm volatile("bar.sync %0, %1;" ::"r"(kBarGo + group), "n"(kGoCount) : "memory");
       if (!*vfail) {
         unsigned char *Ahi = smem + sa * 2 * kTileA, *Alo = Ahi + kTileA;
         const float4 *co = reinterpret_cast<const float4 *>(bring + sb * bst + 2 * btile);
-        const int k0 = ks * kK;
+        const int k0 = (ks0 + ks) * kK;
+        const bool full = m0 + kM <= M_total && k0 + kK <= K_total;
 #pragma unroll
         for (int q = 0; q < kKPerProducer / 4; ++q) {
           uint32_t h[4], l[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int k = kbeg + q * 4 + e;
-            float g = 0.f;
-            if (gm < M_total && k0 + k < K_total) {
-              if (DIR == 0) g = PointKernel<float>::eval(own, own_n, co[k]);
-              else g = PointKernel<float>::eval(co[k], co[kK + k], own);
-            }
+            float g = DIR == 0 ? PointKernel<float>::eval(own, own_n, co[k])
+                               : PointKernel<float>::eval(co[k], co[kK + k], own);
+            if (!full && (gm >= M_total || k0 + k >= K_total)) g = 0.f;
             split_tf32(g, h[e], l[e]);
           }
           const uint32_t off = sw128(row, kbeg + q * 4);
@@ -413,18 +431,20 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
-      asm volatile("bar.sync %0, %1;" ::"n"(kBarAReady), "n"(kGoCount) : "memory");
+      asm volatile("bar.sync %0, %1;" ::"r"(kBarAReady + group), "n"(kGoCount) : "memory");
     }
   } else if (warp == kSchedWarp) {
     // ---------------- scheduler: releases the producers step by step ----------------
     for (int ks = 0; ks < nks; ++ks) {
-      if (lane == 0 && !*vfail) {
-        if (!mbar_wait_one(&bfull[ks % nbs], (ks / nbs) & 1, 0, WL) ||
-            !mbar_wait_one(&aempty[ks % kAStages], ((ks / kAStages) & 1) ^ 1, 0, WL))
-          *s_fail = 1;
+      // two lanes, one poll each: a poll takes hundreds of cycles, and this
+      // warp's are the steps' critical path
+      if (lane < 2 && !*vfail) {
+        uint64_t *bar = lane == 0 ? &bfull[ks % nbs] : &aempty[ks % nas];
+        const uint32_t parity = lane == 0 ? (ks / nbs) & 1 : ((ks / nas) & 1) ^ 1;
+        if (!mbar_wait_one(bar, parity, 0, WL)) *s_fail = 1;
       }
       __syncwarp();
-      asm volatile("bar.sync %0, %1;" ::"n"(kBarGo), "n"(kGoCount) : "memory");
+      asm volatile("bar.sync %0, %1;" ::"r"(kBarGo + ks % kGroups), "n"(kGoCount) : "memory");
     }
   } else if (warp == kLoaderWarp) {
     // ---------------- loader: coordinates + B image by bulk copy ----------------
@@ -440,9 +460,9 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
         }
         unsigned char *bdst = bring + sb * bst;
         unsigned char *cdst = bdst + 2 * btile;
-        const int k0 = ks * kK;
+        const int k0 = (ks0 + ks) * kK;
         mbar_arrive_tx(&bfull[sb], cbytes + bbytes);
-        bulk_g2s(bdst, reinterpret_cast<const unsigned char *>(a.bimg) + (size_t)ks * bbytes, bbytes,
+        bulk_g2s(bdst, reinterpret_cast<const unsigned char *>(a.bimg) + (size_t)(ks0 + ks) * bbytes, bbytes,
                  &bfull[sb]);
         if (DIR == 0) {
           bulk_g2s(cdst, a.ys + k0, cbytes, &bfull[sb]);
@@ -461,17 +481,16 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
     // ---------------- MMA issue ----------------
     const uint32_t idesc = idesc_tf32(a.np);
     for (int ks = 0; ks < nks; ++ks) {
-      const int sa = ks % kAStages, sb = ks % nbs;
+      const int sa = ks % nas, sb = ks % nbs;
       const int kc = ks % kChunk;
       if (lane == 0 && !*vfail) {
-        // the B stage (normally landed long ago), and at a chunk start the
-        // previous chunk folded out of the accumulator
-        if (!mbar_wait_one(&bfull[sb], (ks / nbs) & 1, 0, WL) ||
-            (kc == 0 && ks > 0 && !mbar_wait_one(chunk_free, ((ks / kChunk) - 1) & 1, 0, WL)))
-          *s_fail = 1;
+        // at a chunk start, the previous chunk folded out of the accumulator
+        // (that the B stage has landed is known through the scheduler and the
+        // producers)
+        if (kc == 0 && ks > 0 && !mbar_wait_one(chunk_free, ((ks / kChunk) - 1) & 1, 0, WL)) *s_fail = 1;
       }
       __syncwarp();
-      asm volatile("bar.sync %0, %1;" ::"n"(kBarAReady), "n"(kGoCount) : "memory");
+      asm volatile("bar.sync %0, %1;" ::"r"(kBarAReady + ks % kGroups), "n"(kGoCount) : "memory");
       if (lane == 0 && !*vfail) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t Ahi = smem_u32(smem + sa * 2 * kTileA), Alo = Ahi + kTileA;
@@ -526,12 +545,14 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
           continue;
         }
         if (gm < M_total) {
-          float *o = a.out + (size_t)gm * a.R;
+          const bool split = gridDim.y > 1;
+          float *o = (split ? a.parts + (size_t)blockIdx.y * M_total * a.R : a.out) + (size_t)gm * a.R;
+          const float f = split ? 1.f : a.coef;
 #pragma unroll
           for (int k = 0; k < 32; ++k)
-            if (c0 + k < a.R) o[c0 + k] = a.coef * v[k];
+            if (c0 + k < a.R) o[c0 + k] = f * v[k];
         }
-        if (DIR == 1 && a.part) {
+        if (DIR == 1 && a.part && gridDim.y == 1) {
 #pragma unroll
           for (int k = 0; k < 32; ++k) {
             double d = 0.0;
@@ -554,7 +575,7 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (DIR == 1 && a.part && tid < a.R) {
+  if (DIR == 1 && a.part && gridDim.y == 1 && tid < a.R) {
     a.part[(size_t)blockIdx.x * a.R + tid] =
         *s_fail ? 0.0 : s_red[tid] + s_red[a.R + tid] + s_red[2 * a.R + tid] + s_red[3 * a.R + tid];
   }
@@ -562,6 +583,44 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(tcols) : "memory");
+  }
+}
+
+// out = coef * the sum of the parts in order, with the curvature partials of
+// kSumRows outputs per block (a.part)
+constexpr int kSumRows = 64;
+static __global__ void __launch_bounds__(256) sum_parts_kernel(int M, int R, int nparts, const float *__restrict__ parts,
+                                                               float coef, float *__restrict__ out,
+                                                               const float *__restrict__ pdot, double *__restrict__ part,
+                                                               const int32_t *__restrict__ done)
+{
+  if (done && *done) return;
+  __shared__ double red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i0 = blockIdx.x * kSumRows, c = blockIdx.y * 32 + lane;
+  const size_t stride = (size_t)M * R;
+  double d = 0.0;
+  if (c < R) {
+#pragma unroll 2
+    for (int i = i0 + warp; i < min(M, i0 + kSumRows); i += 8) {
+      const size_t o = (size_t)i * R + c;
+      float v[8], s = 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = q < nparts ? parts[q * stride + o] : 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) s += v[q];
+      s *= coef;
+      out[o] = s;
+      if (part) d += (double)s * (double)pdot[o];
+    }
+  }
+  if (!part) return;
+  red[warp][lane] = d;
+  __syncthreads();
+  if (warp == 0 && c < R) {
+#pragma unroll
+    for (int q = 1; q < 8; ++q) d += red[q][lane];
+    part[(size_t)blockIdx.x * R + c] = d;
   }
 }
 

@@ -122,11 +122,46 @@ static bool use_tc(const Solver &S, int R)
   const int np = (R + 15) / 16 * 16;
   const int K = std::max(S.n, S.nf);
   const size_t need = (size_t)cdiv(K, tc::kK) * 2 * tc::tile_b_bytes(np);
-  // both directions must fit the device's shared memory (true on sm_100a)
-  if (allow_max_smem(tc::pk_tc_kernel<0>, tc::smem_bytes(np, 0)) != MBC_OK ||
-      allow_max_smem(tc::pk_tc_kernel<1>, tc::smem_bytes(np, 1)) != MBC_OK)
-    return false;
+  // both directions must fit the device's shared memory (true on sm_100a);
+  // asked once per solver, the attribute calls cost more than a small product
+  if (!S.tc_smem) {
+    if (allow_max_smem(tc::pk_tc_kernel<0>, tc::kSmemLimit) != MBC_OK ||
+        allow_max_smem(tc::pk_tc_kernel<1>, tc::kSmemLimit) != MBC_OK)
+      return false;
+    S.tc_smem = true;
+  }
   return S.m_bimg.reserve(need) == MBC_OK;
+}
+
+// Parts of the reduction of an M x K tensor-core product.  A CTA fills an SM,
+// so a launch lasts as long as the SM with the most CTAs: with `parts` of the
+// k-steps each, ceil(tiles parts / 148) times steps / parts k-steps of ~1 us,
+// plus ~5 us to start a CTA and, split, ~5 us for the sum of the parts and
+// their round trip.  75 CTAs (9600 outputs) take 7 parts, 500 (64000) 5, which
+// fills their fourth wave.  At most 256 MB of parts.
+static int tc_parts(int M, int K, int R)
+{
+  const double tiles = cdiv(M, tc::kM), steps = cdiv(K, tc::kK);
+  int best = 1;
+  double tbest = 1e300;
+  for (int z = 1; z <= 8; ++z) {
+    const double bytes = 4.0 * z * M * R;
+    if (z > 1 && (steps < 16 * z || bytes > 256e6)) break;
+    const double t = std::ceil(tiles * z / 148.0) * (steps / z + 5.0) + (z > 1 ? 5.0 + 2.0 * bytes / 5e6 : 0.0);
+    if (t < 0.97 * tbest) {
+      tbest = t;
+      best = z;
+    }
+  }
+  return best;
+}
+
+// size the parts' buffer for R columns (before a stream capture)
+static void tc_reserve(const Solver &S, int R)
+{
+  if (!use_tc(S, R)) return;
+  const size_t b = std::max((size_t)tc_parts(S.nf, S.n, R) * S.nf, (size_t)tc_parts(S.n, S.nf, R) * S.n) * R * 4;
+  S.m_tc_parts.reserve(b);  // without it the products run unsplit
 }
 
 template <int DIR>
@@ -158,8 +193,15 @@ static int tc_launch(const Solver &S, int R, const float *vin, float *out, const
                                                               done);
   const int smem = tc::smem_bytes(a.np, DIR);  // allowed by use_tc
   const unsigned grid = cdiv(M, tc::kM);
-  tc::pk_tc_kernel<DIR><<<grid, tc::kThreads, smem, st>>>(a);
-  return (int)grid;
+  int parts = tc_parts(M, K, R);
+  if (parts > 1 && S.m_tc_parts.reserve((size_t)parts * M * R * 4) != MBC_OK) parts = 1;
+  a.parts = (float *)S.m_tc_parts.ptr;
+  tc::pk_tc_kernel<DIR><<<dim3(grid, parts), tc::kThreads, smem, st>>>(a);
+  if (parts == 1) return (int)grid;
+  const unsigned rows = cdiv(M, tc::kSumRows);
+  tc::sum_parts_kernel<<<dim3(rows, cdiv(R, 32)), 256, 0, st>>>(M, R, parts, a.parts, a.coef, out, pdot, part, done);
+  ++S.launches;
+  return (int)rows;
 }
 
 #define MBC_SHAPES(T, X)                                                   \
@@ -739,6 +781,7 @@ static mbc_status pcg_buffers_in(Solver &S, int R, PcgWork<T> &w, DevMem &m, Dev
   w.sc.stall = ii + 2 * R + 4;
   w.sc.drop2 = 0.0;
   w.sc.stall_check = 1;
+  if (sizeof(T) == 4) tc_reserve(S, R);
   return MBC_OK;
 }
 

@@ -49,6 +49,8 @@ struct Solver {
   uint32_t wait_limit = 0;  // polls before a tensor-core kernel's partner wait gives up (0: the default)
   mutable std::bitset<128> p64_smem;  // matvec64.cu kernels whose shared memory is allowed (this solver's device)
   mutable std::bitset<32> dense_smem;  // ... and the dense.cu kernels
+  mutable bool tc_smem = false;  // ... and the FP32 tensor-core kernels
+  mutable DevMem m_tc_parts;     // parts of split FP32 tensor-core products
   mutable DevMem m_bimg;  // packed TF32 hi/lo image of the tensor-core B operand
   // FP64-accurate INT8 matvec: digit planes and exponents of G per direction
   // (0: rows, 1: columns), and the per-launch digit image of the vector block
