@@ -47,9 +47,11 @@
 //   (tensor-memory columns l np .. ): 8 MMAs per 32-byte k-substep instead
 //   of 15.
 //     loader warp  -- bulk-copies the B image of a k-step (ring of 2) and the
-//                     five A plane tiles (ring of 6 single planes);
-//     MMA warp     -- per k-step and plane: waits the tiles, issues the
-//                     MMAs (kind::i8, K = 32, N <= 256 per instruction),
+//                     five A plane tiles (ring of 6 single planes), one lane
+//                     each;
+//     MMA warp     -- per k-step: polls the six tiles at once, and per plane
+//                     that has landed issues the MMAs (kind::i8, K = 32, N <=
+//                     256 per instruction),
 //                     commits the A slot; then the B slot; at a chunk end
 //                     "chunk_full";
 //     8 accumulator warps -- two per tensor-memory lane quarter, half of the
@@ -458,6 +460,9 @@ __host__ __device__ __forceinline__ constexpr uint32_t idesc_i8(int nn)
   return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nn >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
 }
 
+// shared-memory descriptor from its halves (the address sits in the low one)
+__device__ __forceinline__ uint64_t desc_of(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
+
 __device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
                                        uint32_t accumulate)
 {
@@ -579,101 +584,147 @@ __global__ void __launch_bounds__(kThreads, 1) oz_mma_kernel(OzArgs a)
   volatile int *vfail = s_fail;
 
   if (warp == kLoaderWarp) {
-    // ---------------- loader: B image per k-step, then its five A planes ----------------
-    if (lane == 0) {
-      const unsigned char *abase = reinterpret_cast<const unsigned char *>(a.adig);
-      const unsigned char *bbase = reinterpret_cast<const unsigned char *>(a.bimg);
-      int b_issued = 0, a_issued = 0;
-      for (int ks = 0; ks < nks; ++ks) {
-        const int sb = ks % kBSlots;
-        if (*vfail || !tc::mbar_wait_one(&bempty[sb], ((ks / kBSlots) & 1) ^ 1, 32, WL)) {
-          *s_fail = 1;
+    // ---------------- loader: the B image of a k-step and its five A planes ----------------
+    // Lane p < kDigits copies plane p of every k-step, lane kDigits the B
+    // image: the six slots are polled together, and a slot that is free is
+    // filled whatever the others wait for.
+    const bool is_a = lane < kDigits, has = lane <= kDigits;
+    int last = -1;  // the last k-step whose copy this lane issued
+    for (int ks = 0; ks < nks; ++ks) {
+      const int t = ks * kDigits + lane;
+      const int sl = is_a ? t % kASlots : ks % kBSlots, round = is_a ? t / kASlots : ks / kBSlots;
+      uint64_t *empty = is_a ? &aempty[sl] : &bempty[sl], *full = is_a ? &afull[sl] : &bfull[sl];
+      unsigned char *dst = is_a ? aring + sl * kPlaneBytes : bring + sl * BST;
+      const uint32_t bytes = is_a ? kPlaneBytes : BST;
+      const size_t off = is_a ? adig_offset(rt_local, ks, lane, nks) : bimg_offset(grp, ks, nks, NP);
+      const int8_t *src = is_a ? a.adig : a.bimg;
+      bool ok = true;
+      if (has && off + bytes > (is_a ? a.adig_size : a.bimg_size)) {
+        atomicMax(a.err, 4);  // outside its buffer: no copy, fail
+        ok = false;
+      }
+      if (__any_sync(0xffffffffu, !ok || *vfail)) {
+        *s_fail = 1;
+        break;
+      }
+      bool pending = has;
+      for (uint32_t polls = 0; __any_sync(0xffffffffu, pending); ++polls) {
+        if (polls >= WL) {
+          ok = false;
           break;
         }
-        const size_t boff = bimg_offset(grp, ks, nks, NP);
-        if (boff + BST > a.bimg_size) {
-          atomicMax(a.err, 4);  // outside the image: no copy, fail
-          *s_fail = 1;
-          break;
-        }
-        tc::mbar_arrive_tx(&bfull[sb], BST);
-        tc::bulk_g2s(bring + sb * BST, bbase + boff, BST, &bfull[sb]);
-        ++b_issued;
-        bool ok = true;
-        for (int p = 0; p < kDigits; ++p) {
-          const int t = ks * kDigits + p, sa = t % kASlots;
-          const size_t aoff = adig_offset(rt_local, ks, p, nks);
-          if (aoff + kPlaneBytes > a.adig_size) {
-            atomicMax(a.err, 4);  // outside the planes: no copy, fail
-            ok = false;
-            break;
-          }
-          if (!tc::mbar_wait_one(&aempty[sa], ((t / kASlots) & 1) ^ 1, 32, WL)) {
-            ok = false;
-            break;
-          }
-          tc::mbar_arrive_tx(&afull[sa], kPlaneBytes);
-          tc::bulk_g2s(aring + sa * kPlaneBytes, abase + aoff, kPlaneBytes, &afull[sa]);
-          ++a_issued;
-        }
-        if (!ok) {
-          *s_fail = 1;
-          break;
+        if (pending && tc::mbar_test(empty, (round & 1) ^ 1)) {
+          tc::mbar_arrive_tx(full, bytes);
+          tc::bulk_g2s(dst, src + off, bytes, full);
+          last = ks;
+          pending = false;
         }
       }
-      // no copy may still be landing when the CTA exits
-      for (int ks = b_issued > kBSlots ? b_issued - kBSlots : 0; ks < b_issued; ++ks)
-        if (!tc::mbar_wait_one(&bfull[ks % kBSlots], (ks / kBSlots) & 1)) *s_fail = 1;
-      for (int t = a_issued > kASlots ? a_issued - kASlots : 0; t < a_issued; ++t)
-        if (!tc::mbar_wait_one(&afull[t % kASlots], (t / kASlots) & 1)) *s_fail = 1;
+      if (!ok) {
+        *s_fail = 1;
+        break;
+      }
+    }
+    // No copy may still be landing when the CTA exits: lane s < kASlots waits
+    // for the last tile of A slot s, the next kBSlots lanes for the B slots'.
+    // Every lane issued the first `whole` k-steps, those in `more` one more
+    // (an earlier tile of a slot must not be waited for: its phase's parity
+    // reads as incomplete once a later one has completed).
+    int whole = has ? last + 1 : nks;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) whole = min(whole, __shfl_xor_sync(0xffffffffu, whole, o));
+    const uint32_t more = __ballot_sync(0xffffffffu, has && last == whole);
+    if (lane < kASlots) {
+      for (int t = (whole + 1) * kDigits - 1; t >= 0 && t >= (whole - 2) * kDigits; --t)
+        if (t % kASlots == lane && (t / kDigits < whole || (more >> (t % kDigits) & 1u))) {
+          if (!tc::mbar_wait_one(&afull[lane], (t / kASlots) & 1)) *s_fail = 1;
+          break;
+        }
+    } else if (lane < kASlots + kBSlots) {
+      for (int ks = whole; ks >= 0 && ks >= whole - kBSlots; --ks)
+        if (ks % kBSlots == lane - kASlots && (ks < whole || (more >> kDigits & 1u))) {
+          if (!tc::mbar_wait_one(&bfull[lane - kASlots], (ks / kBSlots) & 1)) *s_fail = 1;
+          break;
+        }
     }
   } else if (warp == kMmaWarp) {
     // ---------------- MMA issue ----------------
-    if (lane == 0) {
-      for (int ks = 0; ks < nks; ++ks) {
-        const int kc = ks % kChunkSteps, sb = ks % kBSlots;
-        // the B image, and at a chunk start the previous chunk folded out
-        if (*vfail || !tc::mbar_wait_one(&bfull[sb], (ks / kBSlots) & 1, 0, WL) ||
-            (kc == 0 && ks > 0 && !tc::mbar_wait_one(chunk_free, ((ks / kChunkSteps) - 1) & 1, 32, WL))) {
-          *s_fail = 1;
-          break;
-        }
-        const uint32_t B0 = tc::smem_u32(bring + sb * BST);
-        bool ok = true;
-        for (int p = 0; p < kDigits; ++p) {
-          const int t = ks * kDigits + p, sa = t % kASlots;
-          if (!tc::mbar_wait_one(&afull[sa], (t / kASlots) & 1, 0, WL)) {
+    // Lane p < kDigits polls the A slot of plane p, lane kDigits the B slot and
+    // lane kDigits + 1 "chunk_free" at a chunk start, all at once: a poll costs
+    // about as much as a plane's MMAs, and in the steady state one finds
+    // several planes landed.  Lane 0 issues, from descriptors whose upper
+    // halves are constant.
+    constexpr uint32_t kBBit = 1u << kDigits, kCBit = 1u << (kDigits + 1);
+    const uint32_t dhi = (uint32_t)(tc::desc_sw128(0) >> 32), dlo = (uint32_t)tc::desc_sw128(0);
+    bool ok = true;
+    for (int ks = 0; ks < nks && ok; ++ks) {
+      const int kc = ks % kChunkSteps, sb = ks % kBSlots;
+      uint64_t *bar = &afull[0];
+      uint32_t parity = 0;
+      bool watch = lane < kDigits;
+      if (watch) {
+        const int t = ks * kDigits + lane;
+        bar = &afull[t % kASlots];
+        parity = (t / kASlots) & 1;
+      } else if (lane == kDigits) {
+        bar = &bfull[sb];
+        parity = (ks / kBSlots) & 1;
+        watch = true;
+      } else if (lane == kDigits + 1 && kc == 0 && ks > 0) {
+        bar = chunk_free;
+        parity = ((ks / kChunkSteps) - 1) & 1;
+        watch = true;
+      }
+      uint32_t ready = ~__ballot_sync(0xffffffffu, watch);  // what is not watched needs no wait
+      const uint32_t blo = dlo | (tc::smem_u32(bring + sb * BST) >> 4);
+#pragma unroll
+      for (int p = 0; p < kDigits; ++p) {
+        const uint32_t need = p == 0 ? (1u | kBBit | kCBit) : 1u << p;
+        for (uint32_t polls = 0; (ready & need) != need; ++polls) {
+          if (polls >= WL || __any_sync(0xffffffffu, *vfail)) {  // the same for every lane
             ok = false;
             break;
           }
+          const bool in = watch && !(ready >> lane & 1u) && tc::mbar_test(bar, parity);
+          ready |= __ballot_sync(0xffffffffu, in);
+        }
+        if (!ok) break;
+        __syncwarp();  // orders lane 0 after the polling lanes' acquires
+        const int sa = (ks * kDigits + p) % kASlots;
+        if (lane == 0) {
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t A0 = tc::smem_u32(aring + sa * kPlaneBytes);
-          const int nt = NP * (kDigits - p);  // B rows of planes 0 .. kDigits-1-p
+          const uint32_t alo = dlo | (tc::smem_u32(aring + sa * kPlaneBytes) >> 4);
+          constexpr int NT = NP * kDigits;
+          const int nt = NT - NP * p;  // B rows of planes 0 .. kDigits-1-p
 #pragma unroll
           for (int kk = 0; kk < kKS / 32; ++kk) {
             // the first MMAs of a chunk (plane 0 covers every level column) start from zero
             const uint32_t acc = (kc == 0 && p == 0 && kk == 0) ? 0u : 1u;
-            for (int n0 = 0; n0 < nt; n0 += 256) {
-              const int nn = nt - n0 < 256 ? nt - n0 : 256;
-              mma_i8(tmem + (uint32_t)(p * NP + n0), tc::desc_sw128(A0 + kk * 32),
-                     tc::desc_sw128(B0 + (uint32_t)(n0 / 8) * 1024 + kk * 32), idesc_i8(nn), acc);
+#pragma unroll
+            for (int n0 = 0; n0 < NT; n0 += 256) {
+              if (n0 >= nt) break;
+              mma_i8(tmem + (uint32_t)(p * NP + n0), desc_of(alo + kk * 2, dhi),
+                     desc_of(blo + (uint32_t)(n0 / 8) * 64 + kk * 2, dhi), idesc_i8(nt - n0 < 256 ? nt - n0 : 256), acc);
             }
           }
           tc::mma_commit(&aempty[sa]);
+          if (p == kDigits - 1) {
+            tc::mma_commit(&bempty[sb]);
+            if (kc == kChunkSteps - 1 || ks == nks - 1) tc::mma_commit(chunk_full);
+          }
         }
-        if (!ok) {
-          *s_fail = 1;
-          break;
-        }
-        tc::mma_commit(&bempty[sb]);
-        if (kc == kChunkSteps - 1 || ks == nks - 1) tc::mma_commit(chunk_full);
+        __syncwarp();
       }
+    }
+    if (lane == 0) {
+      if (!ok) *s_fail = 1;
       // after a failure, release the accumulator warps once every MMA issued
       // so far has finished; tensor memory is freed only after that point
       if (*vfail) tc::mma_commit(chunk_full);
       tc::mma_commit(mma_done);
       if (!tc::mbar_wait_one(mma_done, 0)) *s_fail = 1;
     }
+    __syncwarp();
   } else {
     // ---------------- accumulator warps: fold chunks, then the epilogue ----------------
     const int aw = warp - kAccWarp0;  // 0 .. 7

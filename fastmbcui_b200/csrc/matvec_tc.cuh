@@ -181,6 +181,20 @@ __device__ __forceinline__ bool mbar_wait_one(uint64_t *bar, uint32_t parity, ui
   return false;
 }
 
+// whether the phase with the given parity has completed, without waiting
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity)
+{
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // warp-uniform bounded wait: lane 0 polls, the outcome is broadcast and
 // __syncwarp orders the other lanes after lane 0's acquire
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, uint32_t sleep_ns = 0,
