@@ -39,7 +39,7 @@ static void oz_coords(const Solver &S, int DIR, const float4 **xr, const float4 
 }
 
 template <int NPH>
-static void oz_mma_launch(const oz::OzArgs &a, unsigned grid, cudaStream_t st)
+static void oz_mma_launch(const oz::OzArgs &a, dim3 grid, cudaStream_t st)
 {
   oz::oz_mma_kernel<NPH><<<grid, oz::kThreads, oz::smem_bytes(2 * NPH), st>>>(a);
 }
@@ -48,6 +48,45 @@ template <int NPH>
 static mbc_status oz_allow()
 {
   return allow_max_smem(oz::oz_mma_kernel<NPH>, oz::smem_bytes(2 * NPH));
+}
+
+// Parts of the chunks of an M x K product over R columns.  A CTA fills an SM:
+// a launch lasts as long as the SM with the most CTAs, and with a whole
+// reduction per CTA its last wave is often short (188 CTAs on 148 SMs at 24000
+// points and up to 96 columns: two waves for 1.3).  In k-steps of 1 to 2.2 us:
+// ceil(CTAs z / 148) times steps / z, three more to start and drain a CTA, and,
+// split, the sum of the parts and their round trip.  At most 512 MB of parts.
+static int oz_parts(int M, int K, int R)
+{
+  const double ctas = (double)oz::row_tiles(M) * oz::groups_for(R), steps = oz::nks_for(K);
+  const double us = 1.0 + 0.0125 * oz::np_for(R);
+  int best = 1;
+  double tbest = 1e300;
+  for (int z = 1; z <= 8 && z <= oz::nchunks_for(K); ++z) {
+    const double bytes = 8.0 * z * M * R;
+    if (z > 1 && bytes > 512e6) break;
+    const double per = (double)cdiv(oz::nchunks_for(K), z) * oz::kChunkSteps;  // whole chunks
+    const double t = us * std::ceil(ctas * z / 148.0) * (std::min(per, steps) + 3.0) +
+                     (z > 1 ? 6.0 + 2.0 * bytes / 5e6 : 0.0);
+    if (t < 0.97 * tbest) {
+      tbest = t;
+      best = z;
+    }
+  }
+  return best;
+}
+
+// bytes of parts any product of at most R columns takes
+static size_t oz_parts_bytes(const Solver &S, int R)
+{
+  size_t b = 0;
+  for (int r = 1; r <= R; ++r)
+    for (int dir = 0; dir < 2; ++dir) {
+      const int M = dir == 0 ? S.nf : S.n, K = dir == 0 ? S.n : S.nf;
+      const int z = oz_parts(M, K, r);
+      if (z > 1) b = std::max(b, (size_t)8 * z * M * r);
+    }
+  return b;
 }
 
 // pack the vector block, then the MMA kernel; returns the row tiles (the
@@ -87,9 +126,12 @@ static int oz_launch(const Solver &S, int R, const double *vin, double *out, con
   a.done = done;
   a.err = (int32_t *)S.m_err.ptr;
   a.wait_limit = S.wait_limit;
+  int parts = S.oz_slab ? 1 : oz_parts(M, K, R);
+  if ((size_t)8 * parts * M * R > S.m_oz_parts.bytes) parts = 1;
+  a.parts = (double *)S.m_oz_parts.ptr;
   auto mma = [&](int rt0, int tiles) {
     a.rt0 = rt0;
-    const unsigned grid = (unsigned)tiles * (unsigned)groups;
+    const dim3 grid((unsigned)tiles * (unsigned)groups, (unsigned)parts);
     switch (np) {
       case 16: oz_mma_launch<8>(a, grid, st); break;
       case 32: oz_mma_launch<16>(a, grid, st); break;
@@ -103,6 +145,13 @@ static int oz_launch(const Solver &S, int R, const double *vin, double *out, con
   if (!S.oz_slab) {
     mma(0, tiles);
     S.launches += 2;
+    if (parts > 1) {
+      const unsigned rows = cdiv(M, tc::kSumRows);
+      tc::sum_parts_kernel<double><<<dim3(rows, cdiv(R, 32)), 256, 0, st>>>(M, R, parts, a.parts, a.coef, out, pdot, part,
+                                                                           done);
+      ++S.launches;
+      return (int)rows;
+    }
   } else {
     // the planes of each slab of rows, then its products
     const int per = S.oz_slab_tiles[DIR];
@@ -235,6 +284,10 @@ mbc_status mbc::Solver::ensure_oz(cudaStream_t st, int R)
   const int K = std::max(n, nf);
   MBC_TRY(m_oz_b.reserve(oz::bimg_bytes(K, R)));
   MBC_TRY(m_oz_bexp.reserve(sizeof(int32_t) * oz::bexp_count(K, R)));
+  if (!oz_slab && R > oz_parts_R) {  // sized before any capture; without it products run unsplit
+    m_oz_parts.reserve(oz_parts_bytes(*this, R));
+    oz_parts_R = R;
+  }
   return MBC_OK;
 }
 

@@ -505,6 +505,7 @@ struct OzArgs {
   size_t aexp_size, bexp_size;  // entries
   int rt0;              // first row tile of this launch (slab); adig holds the slab's planes
   double *out;          // M x R
+  double *parts;        // gridDim.y > 1: [part][M][R] sums of the parts of the chunks, without coef
   int M, K, R, groups;  // outputs, reduction length, columns, column groups
   double coef;
   const double *pdot;   // columns: p (M x R) for the curvature partials, or NULL
@@ -550,8 +551,12 @@ __global__ void __launch_bounds__(kThreads, 1) oz_mma_kernel(OzArgs a)
   const int rt_local = blockIdx.x / a.groups, grp = blockIdx.x - rt_local * a.groups;
   const int rt = a.rt0 + rt_local;  // global row tile: exponents, outputs, partials
   const int m0 = rt * kM;
-  const int nks = nks_for(a.K);
-  const int nchunks = nchunks_for(a.K);
+  // this CTA's part of the chunks: the loops run over ks - ks_off, c - cb
+  const int nks_all = nks_for(a.K), nchunks_all = nchunks_for(a.K);
+  const int cb = (int)((int64_t)nchunks_all * blockIdx.y / gridDim.y);
+  const int nchunks = (int)((int64_t)nchunks_all * (blockIdx.y + 1) / gridDim.y) - cb;
+  const int ks_off = cb * kChunkSteps;
+  const int nks = min(nks_all, (cb + nchunks) * kChunkSteps) - ks_off;
   // the partner-wait limit, read from the parameter bank at each use
 #define WL (a.wait_limit ? a.wait_limit : kWaitLimit)
 
@@ -596,7 +601,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_mma_kernel(OzArgs a)
       uint64_t *empty = is_a ? &aempty[sl] : &bempty[sl], *full = is_a ? &afull[sl] : &bfull[sl];
       unsigned char *dst = is_a ? aring + sl * kPlaneBytes : bring + sl * BST;
       const uint32_t bytes = is_a ? kPlaneBytes : BST;
-      const size_t off = is_a ? adig_offset(rt_local, ks, lane, nks) : bimg_offset(grp, ks, nks, NP);
+      const size_t off = is_a ? adig_offset(rt_local, ks_off + ks, lane, nks_all) : bimg_offset(grp, ks_off + ks, nks_all, NP);
       const int8_t *src = is_a ? a.adig : a.bimg;
       bool ok = true;
       if (has && off + bytes > (is_a ? a.adig_size : a.bimg_size)) {
@@ -748,14 +753,14 @@ __global__ void __launch_bounds__(kThreads, 1) oz_mma_kernel(OzArgs a)
       // the check covers the whole CTA's exponents, so every accumulator
       // thread takes the same branch (a partial exit would strand the others
       // at the named barrier)
-      if (aexp_index(rt, c, kM - 1, nchunks) >= a.aexp_size ||
-          bexp_index(grp, c, 0, nchunks, NP) + NP > a.bexp_size) {
+      if (aexp_index(rt, cb + c, kM - 1, nchunks_all) >= a.aexp_size ||
+          bexp_index(grp, cb + c, 0, nchunks_all, NP) + NP > a.bexp_size) {
         if (aw == 0 && lane == 0) atomicMax(a.err, 4);  // no fold, fail (the MMA warp's wait expires)
         ok = false;
         break;
       }
-      const int ea = a.aexp[aexp_index(rt, c, row, nchunks)];
-      const int32_t *eb = a.bexp + bexp_index(grp, c, c0, nchunks, NP);
+      const int ea = a.aexp[aexp_index(rt, cb + c, row, nchunks_all)];
+      const int32_t *eb = a.bexp + bexp_index(grp, cb + c, c0, nchunks_all, NP);
 #pragma unroll
       for (int g = 0; g < NPH / 8; ++g) {
         int32_t v[kLevels][8];
@@ -777,12 +782,14 @@ __global__ void __launch_bounds__(kThreads, 1) oz_mma_kernel(OzArgs a)
     if (!ok) *s_fail = 1;
     const int col0 = grp * NP + c0;
     if (ok && gm < a.M) {
-      double *o = a.out + (size_t)gm * a.R + col0;
+      const bool split = gridDim.y > 1;
+      double *o = (split ? a.parts + (size_t)blockIdx.y * a.M * a.R : a.out) + (size_t)gm * a.R + col0;
+      const double f = split ? 1.0 : a.coef;
 #pragma unroll
       for (int k = 0; k < NPH; ++k)
-        if (col0 + k < a.R) o[k] = a.coef * sum[k];
+        if (col0 + k < a.R) o[k] = f * sum[k];
     }
-    if (a.part) {
+    if (a.part && gridDim.y == 1) {
 #pragma unroll
       for (int k = 0; k < NPH; ++k) {
         double d = 0.0;
@@ -795,7 +802,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_mma_kernel(OzArgs a)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (a.part && tid < NP && grp * NP + tid < a.R) {
+  if (a.part && gridDim.y == 1 && tid < NP && grp * NP + tid < a.R) {
     a.part[(size_t)rt * a.R + grp * NP + tid] =
         *s_fail ? 0.0 : s_red[tid] + s_red[NP + tid] + s_red[2 * NP + tid] + s_red[3 * NP + tid];
   }

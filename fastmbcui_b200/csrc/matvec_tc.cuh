@@ -603,10 +603,10 @@ __global__ void __launch_bounds__(kThreads, 1) pk_tc_kernel(TcArgs a)
 // out = coef * the sum of the parts in order, with the curvature partials of
 // kSumRows outputs per block (a.part)
 constexpr int kSumRows = 64;
-static __global__ void __launch_bounds__(256) sum_parts_kernel(int M, int R, int nparts, const float *__restrict__ parts,
-                                                               float coef, float *__restrict__ out,
-                                                               const float *__restrict__ pdot, double *__restrict__ part,
-                                                               const int32_t *__restrict__ done)
+template <typename T>
+static __global__ void __launch_bounds__(256) sum_parts_kernel(int M, int R, int nparts, const T *__restrict__ parts,
+                                                               T coef, T *__restrict__ out, const T *__restrict__ pdot,
+                                                               double *__restrict__ part, const int32_t *__restrict__ done)
 {
   if (done && *done) return;
   __shared__ double red[8][32];
@@ -618,9 +618,9 @@ static __global__ void __launch_bounds__(256) sum_parts_kernel(int M, int R, int
 #pragma unroll 2
     for (int i = i0 + warp; i < min(M, i0 + kSumRows); i += 8) {
       const size_t o = (size_t)i * R + c;
-      float v[8], s = 0.f;
+      T v[8], s = T(0);
 #pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = q < nparts ? parts[q * stride + o] : 0.f;
+      for (int q = 0; q < 8; ++q) v[q] = q < nparts ? parts[q * stride + o] : T(0);
 #pragma unroll
       for (int q = 0; q < 8; ++q) s += v[q];
       s *= coef;

@@ -199,7 +199,7 @@ static int tc_launch(const Solver &S, int R, const float *vin, float *out, const
   tc::pk_tc_kernel<DIR><<<dim3(grid, parts), tc::kThreads, smem, st>>>(a);
   if (parts == 1) return (int)grid;
   const unsigned rows = cdiv(M, tc::kSumRows);
-  tc::sum_parts_kernel<<<dim3(rows, cdiv(R, 32)), 256, 0, st>>>(M, R, parts, a.parts, a.coef, out, pdot, part, done);
+  tc::sum_parts_kernel<float><<<dim3(rows, cdiv(R, 32)), 256, 0, st>>>(M, R, parts, a.parts, a.coef, out, pdot, part, done);
   ++S.launches;
   return (int)rows;
 }

@@ -56,6 +56,8 @@ struct Solver {
   // (0: rows, 1: columns), and the per-launch digit image of the vector block
   DevMem m_oz_a[2], m_oz_aexp[2];
   mutable DevMem m_oz_b, m_oz_bexp;
+  DevMem m_oz_parts;   // parts of split INT8 products of up to oz_parts_R columns
+  int oz_parts_R = 0;
   // the reduction axes of the INT8 planes walk the points in Morton order:
   // m_oz_q[0][k] = plan position of the k-th source (K direction), m_oz_q[1][k]
   // = the k-th collocation row (K^T direction); the coordinates in that order
