@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(kThreads) block_update_kernel(int n, int k, in
 // kPackedDim; above that the kernels work on the global copy (L1 / L2).  The
 // arithmetic and its order are the same either way.
 constexpr int kPackedDim = 208;  // 208 * 209 / 2 doubles = 169.8 KB
+constexpr int kOrthMax = 512;    // widest block
 constexpr int kSolveWarps = 8;   // columns (one warp each) per block of the column-parallel solves
 
 __host__ __device__ constexpr size_t packed_len(int k) { return (size_t)k * (k + 1) / 2; }
@@ -184,30 +185,34 @@ __device__ __forceinline__ void stage_lower(int k, const double *src, int ld, do
 __global__ void __launch_bounds__(kSmallThreads) chol_kernel(int k, double *Gg, int ldg, int32_t *flag, int packed)
 {
   extern __shared__ double sm[];
-  __shared__ int bad;
-  if (threadIdx.x == 0) bad = 0;
+  __shared__ double s_col[kOrthMax];
   if (packed) stage_lower(k, Gg, ldg, sm);
   const Lower G{packed ? sm : Gg, ldg, packed};
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   __syncthreads();
+  bool bad = false;  // the same in every thread
   for (int j = 0; j < k; ++j) {
-    if (threadIdx.x == 0) {
-      const double d = G(j, j);
-      if (!(d > 0.0)) bad = 1;
-      G(j, j) = d > 0.0 ? sqrt(d) : 1.0;
+    // every thread has the pivot; the scaled column goes to its own array, so
+    // that two barriers a step suffice
+    const double d = G(j, j);
+    bad = !(d > 0.0);
+    if (bad) break;
+    const double root = sqrt(d);
+    for (int i = j + 1 + threadIdx.x; i < k; i += blockDim.x) {
+      const double v = G(i, j) / root;
+      G(i, j) = v;
+      s_col[i] = v;
     }
     __syncthreads();
-    if (bad) break;
-    const double djj = G(j, j);
-    for (int i = j + 1 + threadIdx.x; i < k; i += blockDim.x) G(i, j) /= djj;
-    __syncthreads();
+    if (threadIdx.x == 0) G(j, j) = root;
     // trailing update of the lower triangle, one warp per row
     for (int i = j + 1 + warp; i < k; i += nw) {
-      const double gij = G(i, j);
-      for (int l = j + 1 + lane; l <= i; l += 32) G(i, l) -= gij * G(l, j);
+      const double gij = s_col[i];
+      for (int l = j + 1 + lane; l <= i; l += 32) G(i, l) -= gij * s_col[l];
     }
     __syncthreads();
   }
+  __syncthreads();
   if (packed) {
     for (int i = warp; i < k; i += nw)
       for (int l = lane; l <= i; l += 32) Gg[(size_t)i * ldg + l] = G(i, l);
@@ -215,12 +220,56 @@ __global__ void __launch_bounds__(kSmallThreads) chol_kernel(int k, double *Gg, 
   if (threadIdx.x == 0 && bad && flag) *flag = 1;
 }
 
+// Substitutions with a lower factor L (k <= 32 kRegTiles) for one column per
+// warp, the column in registers: entry 32 q + lane in x[q].  A step is one
+// shuffle, one multiplication with the inverse diagonal and the lanes'
+// updates, whose L values don't depend on it; with the column in shared memory
+// and divisions a step took twice as long (24000 points, blocks from 192
+// columns down: chol_solve_kernel 73 -> 38 us on average, the step's 33).
+constexpr int kRegTiles = 7;
+__device__ __forceinline__ void forward_sub(int k, const Lower &L, const double *invd, double (&x)[kRegTiles])
+{
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int qj = 0; qj < kRegTiles; ++qj) {
+    const int jm = min(32, k - 32 * qj);
+    for (int jj = 0; jj < jm; ++jj) {
+      const int j = 32 * qj + jj;
+      const double y = __shfl_sync(0xffffffffu, x[qj], jj) * invd[j];
+      if (lane == jj) x[qj] = y;
+#pragma unroll
+      for (int q = qj; q < kRegTiles; ++q) {
+        const int i = 32 * q + lane;
+        if (i > j && i < k) x[q] -= L(i, j) * y;
+      }
+    }
+  }
+}
+// ... from step j0 down with L^T
+__device__ __forceinline__ void backward_sub(int j0, const Lower &L, const double *invd, double (&x)[kRegTiles])
+{
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int qj = kRegTiles - 1; qj >= 0; --qj) {
+    for (int jj = min(31, j0 - 32 * qj); jj >= 0; --jj) {
+      const int j = 32 * qj + jj;
+      const double y = __shfl_sync(0xffffffffu, x[qj], jj) * invd[j];
+      if (lane == jj) x[qj] = y;
+#pragma unroll
+      for (int q = 0; q <= qj; ++q) {
+        const int i = 32 * q + lane;
+        if (i < j) x[q] -= L(j, i) * y;
+      }
+    }
+  }
+}
+
 // B (k x m, ldb) <- sgn * (L L^T)^{-1} B for the lower factor L of
 // chol_kernel (lower triangle of Lg, ldg).  One warp per column of B,
 // kSolveWarps columns per block, grid cdiv(m, kSolveWarps): forward then
 // backward substitution in the column-oriented order, the column held in
-// shared memory.  Dynamic shared memory: kSolveWarps * k doubles, plus
-// packed_len(k) with packed (L staged).  Nothing is done when *skip is set
+// registers (k <= 32 kRegTiles) or shared memory.  Dynamic shared memory:
+// (kSolveWarps + 1) k doubles, plus packed_len(k) with packed (L staged).  Nothing is done when *skip is set
 // (the factorization failed).
 __global__ void __launch_bounds__(kSolveWarps * 32) chol_solve_kernel(int k, const double *Lg, int ldg, int m,
                                                                       double *B, int ldb, double sgn,
@@ -229,18 +278,32 @@ __global__ void __launch_bounds__(kSolveWarps * 32) chol_solve_kernel(int k, con
   extern __shared__ double sm[];
   if (skip && *skip) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double *Lp = sm + (size_t)kSolveWarps * k;
+  double *invd = sm + (size_t)kSolveWarps * k;
+  double *Lp = invd + k;
+  for (int i = threadIdx.x; i < k; i += blockDim.x) invd[i] = 1.0 / Lg[(size_t)i * ldg + i];
   if (packed) stage_lower(k, Lg, ldg, Lp);
+  else __syncthreads();
   const Lower L{packed ? Lp : const_cast<double *>(Lg), ldg, packed};
   const int c = blockIdx.x * kSolveWarps + warp;
   if (c >= m) return;
+  if (k <= 32 * kRegTiles) {
+    double r[kRegTiles];
+#pragma unroll
+    for (int q = 0; q < kRegTiles; ++q) r[q] = 32 * q + lane < k ? B[(size_t)(32 * q + lane) * ldb + c] : 0.0;
+    forward_sub(k, L, invd, r);
+    backward_sub(k - 1, L, invd, r);
+#pragma unroll
+    for (int q = 0; q < kRegTiles; ++q)
+      if (32 * q + lane < k) B[(size_t)(32 * q + lane) * ldb + c] = sgn * r[q];
+    return;
+  }
   double *x = sm + (size_t)warp * k;
   for (int i = lane; i < k; i += 32) x[i] = B[(size_t)i * ldb + c];
   __syncwarp();
   // forward: L y = b.  Every lane reads x[j] before the __syncwarp; lane 0
   // stores y_j after it (x[j] is read again only in the backward pass).
   for (int j = 0; j < k; ++j) {
-    const double yj = x[j] / L(j, j);
+    const double yj = x[j] * invd[j];
     for (int i = j + 1 + lane; i < k; i += 32) x[i] -= L(i, j) * yj;
     __syncwarp();
     if (lane == 0) x[j] = yj;
@@ -248,7 +311,7 @@ __global__ void __launch_bounds__(kSolveWarps * 32) chol_solve_kernel(int k, con
   __syncwarp();
   // backward: L^T x = y
   for (int j = k - 1; j >= 0; --j) {
-    const double xj = x[j] / L(j, j);
+    const double xj = x[j] * invd[j];
     for (int i = lane; i < j; i += 32) x[i] -= L(j, i) * xj;
     __syncwarp();
     if (lane == 0) x[j] = xj;
@@ -256,8 +319,6 @@ __global__ void __launch_bounds__(kSolveWarps * 32) chol_solve_kernel(int k, con
   __syncwarp();
   for (int i = lane; i < k; i += 32) B[(size_t)i * ldb + c] = sgn * x[i];
 }
-
-constexpr int kOrthMax = 512;  // widest block orth_factor_kernel takes
 
 // Rank-revealing Cholesky of the m x m Gram matrix W (row-major, ld; lower
 // triangle read, overwritten by the factor) of a block V (m <= kOrthMax).
@@ -281,6 +342,7 @@ __global__ void __launch_bounds__(kSmallThreads) orth_factor_kernel(int m, doubl
   __shared__ int s_r;
   __shared__ double s_dmax;
   __shared__ double s_scale[kOrthMax];
+  __shared__ double s_col[kOrthMax];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const Lower W{packed ? sm : Wg, ldg, packed};
   for (int i = threadIdx.x; i < m; i += blockDim.x) {
@@ -310,51 +372,44 @@ __global__ void __launch_bounds__(kSmallThreads) orth_factor_kernel(int m, doubl
   }
   const double thr = drop > 0.0 ? drop * drop * s_dmax : 0.0;
   // pivoted Cholesky of the symmetric matrix on its lower triangle, rows and
-  // columns swapped in place
+  // columns swapped in place; three barriers a step: the pivot (one warp), the
+  // swap with the scaled column, the trailing update.  Bound by the barriers
+  // of 1024 threads: 379 -> 176 us on average over a step's 17 factorizations
   for (int j = 0; j < m; ++j) {
-    // pivot: the largest remaining diagonal (lowest index on ties)
-    double best = -1.0;
-    int bi = j;
-    for (int i = j + threadIdx.x; i < m; i += blockDim.x) {
-      const double d = W(i, i);
-      if (d > best) {
-        best = d;
-        bi = i;
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) {
-        best = ob;
-        bi = oi;
-      }
-    }
-    if (lane == 0) {
-      s_val[warp] = best;
-      s_idx[warp] = bi;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double b = -1.0;
-      int p = j;
-      for (int w = 0; w < nw; ++w)
-        if (s_val[w] > b || (s_val[w] == b && s_idx[w] < p)) {
-          b = s_val[w];
-          p = s_idx[w];
+    if (warp == 0) {
+      // pivot: the largest remaining diagonal (lowest index on ties)
+      double best = -1.0;
+      int bi = j;
+      for (int i = j + lane; i < m; i += 32) {
+        const double d = W(i, i);
+        if (d > best) {
+          best = d;
+          bi = i;
         }
-      s_idx[0] = p;
-      s_val[0] = b;
-      if (!(b > thr)) s_r = j;
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ob > best || (ob == best && oi < bi)) {
+          best = ob;
+          bi = oi;
+        }
+      }
+      if (lane == 0) {
+        s_idx[0] = bi;
+        s_val[0] = best;
+        if (!(best > thr)) s_r = j;
+      }
     }
     __syncthreads();
     if (s_r == j) break;
     const int p = s_idx[0];
-    if (p != j) {
-      // swap rows and columns j < p of the symmetric matrix, on the lower
-      // triangle: each x other than j and p pairs two entries; (p, j) stays
-      for (int x = threadIdx.x; x < m; x += blockDim.x) {
-        if (x == p) continue;
+    const double root = sqrt(s_val[0]);
+    // Swap rows and columns j < p of the symmetric matrix, on the lower
+    // triangle: each x other than j and p pairs two entries; (p, j) stays.
+    // Thread x also holds entry (x, j) of the new order and scales it.
+    for (int x = threadIdx.x; x < m; x += blockDim.x) {
+      if (p != j && x != p) {
         double *e1, *e2;
         if (x == j) {
           e1 = &W(j, j);
@@ -373,22 +428,23 @@ __global__ void __launch_bounds__(kSmallThreads) orth_factor_kernel(int m, doubl
         *e1 = *e2;
         *e2 = t;
       }
-      if (threadIdx.x == 0) {
-        const int32_t q = perm[j];
-        perm[j] = perm[p];
-        perm[p] = q;
+      if (x > j) {
+        const double v = W(x, j) / root;
+        W(x, j) = v;
+        s_col[x] = v;
       }
-      __syncthreads();
     }
-    if (threadIdx.x == 0) W(j, j) = sqrt(W(j, j));
+    if (threadIdx.x == 0 && p != j) {
+      const int32_t q = perm[j];
+      perm[j] = perm[p];
+      perm[p] = q;
+    }
     __syncthreads();
-    const double djj = W(j, j);
-    for (int i = j + 1 + threadIdx.x; i < m; i += blockDim.x) W(i, j) /= djj;
-    __syncthreads();
+    if (threadIdx.x == 0) W(j, j) = root;
     // trailing update of the lower triangle, one warp per row
     for (int i = j + 1 + warp; i < m; i += nw) {
-      const double wij = W(i, j);
-      for (int l = j + 1 + lane; l <= i; l += 32) W(i, l) -= wij * W(l, j);
+      const double wij = s_col[i];
+      for (int l = j + 1 + lane; l <= i; l += 32) W(i, l) -= wij * s_col[l];
     }
     __syncthreads();
   }
@@ -414,16 +470,34 @@ __global__ void __launch_bounds__(kSolveWarps * 32) orth_t_kernel(int m, const d
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = *rank;
   if (blockIdx.x * kSolveWarps >= r) return;
-  double *Lp = sm + (size_t)kSolveWarps * m;
+  double *invd = sm + (size_t)kSolveWarps * m;
+  double *Lp = invd + m;
+  for (int i = threadIdx.x; i < r; i += blockDim.x) invd[i] = 1.0 / Wg[(size_t)i * ldg + i];
   if (packed) stage_lower(r, Wg, ldg, Lp);
+  else __syncthreads();
   const Lower L{packed ? Lp : const_cast<double *>(Wg), ldg, packed};
   const int c = blockIdx.x * kSolveWarps + warp;
   if (c >= r) return;
+  if (m <= 32 * kRegTiles) {
+    double v[kRegTiles];
+#pragma unroll
+    for (int q = 0; q < kRegTiles; ++q) v[q] = 32 * q + lane == c ? 1.0 : 0.0;
+    backward_sub(c, L, invd, v);
+#pragma unroll
+    for (int q = 0; q < kRegTiles; ++q) {
+      const int i = 32 * q + lane;
+      if (i < m) {
+        const int pi = perm[i];
+        T[(size_t)pi * ldt + c] = v[q] * scale[pi];
+      }
+    }
+    return;
+  }
   double *x = sm + (size_t)warp * m;
   for (int i = lane; i < m; i += 32) x[i] = i == c ? 1.0 : 0.0;
   __syncwarp();
   for (int j = c; j >= 0; --j) {
-    const double xj = x[j] / L(j, j);
+    const double xj = x[j] * invd[j];
     for (int i = lane; i < j; i += 32) x[i] -= L(j, i) * xj;
     __syncwarp();
     if (lane == 0) x[j] = xj;

@@ -1120,7 +1120,7 @@ static mbc_status run_block_pcg(Solver &S, int R, PcgWork<double> &w, const LT *
   // per warp
   auto packed = [](int k) -> int { return k <= blk::kPackedDim; };
   auto smem_fac = [&](int k) -> size_t { return packed(k) ? sizeof(double) * blk::packed_len(k) : 0; };
-  auto smem_sol = [&](int k) -> size_t { return sizeof(double) * (size_t)blk::kSolveWarps * k + smem_fac(k); };
+  auto smem_sol = [&](int k) -> size_t { return sizeof(double) * (size_t)(blk::kSolveWarps + 1) * k + smem_fac(k); };
   const size_t smem_sol_max = std::max(smem_sol(blk::kPackedDim), smem_sol(blk::kOrthMax));
   MBC_TRY(allow_max_smem(blk::chol_kernel, smem_fac(blk::kPackedDim)));
   MBC_TRY(allow_max_smem(blk::orth_factor_kernel, smem_fac(blk::kPackedDim)));
