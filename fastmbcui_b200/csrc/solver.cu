@@ -701,7 +701,8 @@ static bool reduce_in_place(int nblk, int R) { return (int64_t)cdiv(nblk, 32) * 
 
 // The two halves of the preconditioner, z = L (L^T r); with `part` the second
 // forms the partials of r . z and, for mode RED_BETA, their reduction.
-// Warps per row: as many as keep ~16 warps per SM busy in small scenes.
+// Warps per row: as many as keep ~16 warps per SM busy in small scenes.  The
+// grid is one wave of resident blocks: six of 256 threads at 40 registers.
 struct PrecondShape {
   dim3 grid;
   int cx, wpr;
@@ -714,7 +715,7 @@ static PrecondShape precond_shape(int n, int R)
   const unsigned gy = cdiv(R, s.cx);
   s.wpr = 1;
   while (s.wpr < 8 && (int64_t)n * gy * s.wpr < 16 * 148) s.wpr <<= 1;
-  s.grid = dim3(std::min<unsigned>(cdiv(n, 8 / s.wpr), std::max(8u * 148u / gy, 1u)), gy);
+  s.grid = dim3(std::min<unsigned>(cdiv(n, 8 / s.wpr), std::max(6u * 148u / gy, 1u)), gy);
   return s;
 }
 template <typename T, typename LT>
