@@ -561,7 +561,7 @@ def _matvec_roofline(st, nf, n, R, matvec, fp64_matvec="simt"):
     if fp64_matvec == "int8" and n64:
         tops = 2.0 * 15 * nf * n * c64 / sec64 / 1e12
         gbs = 5.0 * nf * n * n64 / sec64 / 1e9
-        fp64.update({"kernel": "oz_gather + oz_pack_b_kernel + oz_mma_kernel (tcgen05 kind::i8, 5-digit slicing)",
+        fp64.update({"kernel": "oz_pack_b_kernel + oz_mma_kernel (tcgen05 kind::i8, 5-digit slicing)",
                      "achieved_int8_tops": round(tops, 1), "int8_peak_tops": 2 * bf16,
                      "frac_of_int8": round(tops / (2 * bf16), 4), "plane_gbs": round(gbs, 1),
                      "frac_of_hbm": round(gbs / hbm, 4)})
@@ -575,7 +575,7 @@ def _matvec_roofline(st, nf, n, R, matvec, fp64_matvec="simt"):
                 "kernel": fp64["kernel"], "launch_ms": round(ms64, 3),
                 "peak_source": f"INT8 dense = 2 x bf16 dense ({src}); HBM {hbm} GB/s ({src})",
                 "fp64_matvec": fp64, "tensor_matvec": tc}
-    fp64.update({"kernel": "pk_rows_kernel / pk_cols_kernel<double> (FP64 SIMT)", "fp64_nominal_tflops": 37.0,
+    fp64.update({"kernel": "p64::pk64_kernel (FP64 mma.sync)", "fp64_nominal_tflops": 37.0,
                  "frac_of_fp64_nominal": round(a64 / 37.0, 4)})
     dom64 = t64 >= t32
     ach, ms = (a64, ms64) if dom64 else (a32, ms32)

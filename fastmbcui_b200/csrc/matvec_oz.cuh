@@ -33,7 +33,7 @@
 // the recomputed residual) in 4 % more iterations than the FP64 operator.
 //
 // G is evaluated with PointKernel<double>::eval, the function the FP64
-// CUDA-core kernels use, so the digits encode the same FP64 values.  G does
+// kernels use, so the digits encode the same FP64 values.  G does
 // not change while a solver lives, so its digit planes are built once per
 // solver and direction (oz_digits_kernel: 5 bytes per matrix entry, stored
 // in the shared-memory image the MMA reads); a matvec packs only the vector

@@ -1471,7 +1471,7 @@ mbc_status Solver::solve_plain(int R, const void *rhs, int32_t rhs_dt, void *X, 
       // The decision residual is FP64-accurate: the products whose inputs
       // cancel against the right-hand side (K x for the forward residual
       // f - K x, both products of the adjoint's b - K^T K x) run on the FP64
-      // CUDA-core kernels.  K x of the solution carries the INT8 operator's
+      // kernels.  K x of the solution carries the INT8 operator's
       // ~1e-9 relative error against a least-squares residual f - K x ~1e-7
       // |f|; K^T of that residual on the INT8 matvec agrees with FP64 to
       // ~10 digits (measured), so it stays there.  Only |b| (a norm) uses
@@ -1535,7 +1535,7 @@ mbc_status Solver::solve_plain(int R, const void *rhs, int32_t rhs_dt, void *X, 
                                                                              (const T *)fm.ptr, (T *)fsub.ptr);
         launches += 3;
         MBC_CKL();
-        // the last restart runs on the FP64 CUDA-core matvec: a column the
+        // the last restart runs on the FP64 matvec: a column the
         // INT8 operator's ~1e-9 product error keeps above tol (near-singular
         // kernels: sources close to a thin body) converges there, at a cost
         // proportional to the few columns left
@@ -1590,7 +1590,7 @@ mbc_status Solver::solve_plain(int R, const void *rhs, int32_t rhs_dt, void *X, 
 mbc_status Solver::true_residual(int R, const void *F, int32_t f_dt, const void *X, int32_t x_dt,
                                  mbc_solve_stats *stats, cudaStream_t st)
 {
-  // always the FP64 CUDA-core kernels, whatever FP64 matvec the solves use
+  // always the FP64 kernels, whatever FP64 matvec the solves use
   struct Restore {
     Solver &S;
     int32_t impl;

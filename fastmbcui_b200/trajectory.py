@@ -14,7 +14,7 @@ Precision modes (``mode``):
            Cholesky cancels are refactored in FP64); the PCG recursion,
            dot products and scalars in FP64; the matvecs FP64-accurate
            (``fp64_matvec="int8"``: exact digit slices on the INT8 tensor
-           cores, or "simt": FP64 CUDA cores).
+           cores, or "simt": the FP64 kernels).
   "fp64"   the plain method: FP64 factor and FP64 PCG.
   "fp32-replace"  FP32 recursion (tensor-core 3xTF32 matvec) with FP64
            residual replacement and an FP64 polish of stagnating columns.

@@ -128,7 +128,7 @@ typedef struct {
    * (vertices V[faces[f][0..2]]) seen from source y_j, evaluated on the fly
    * (the dense matrix mbc_mesh_assemble writes, never stored).  nf = faces;
    * faces: device nf x 3 int32; V: device n_vert x 3; y: device n x 3.
-   * FP64 and FP32 CUDA-core matvecs (no tensor-core or INT8 form). */
+   * FP64 and FP32 matvecs (no tcgen05 or INT8 form). */
   const float *V;
   const int32_t *faces;
   int32_t n_vert;
@@ -165,8 +165,8 @@ mbc_status mbc_solver_get_factor(const mbc_solver *s, double *lval_host, double 
  * shapes change the order of the Gram sums (results agree to rounding), not
  * the method.  In FP32 factors, supernodes with tc_min_ns <= n_s <= 192 form
  * Theta_s on the tensor cores (tcgen05, 3xTF32 with FP32 chunk sums) before
- * their class kernel factors it; 0 keeps every Gram on the CUDA cores.  FP64
- * factors and the FP64 retries always use the CUDA cores.  No counterpart in
+ * their class kernel factors it; 0 keeps every Gram off them.  FP64
+ * factors and the FP64 retries never use them.  No counterpart in
  * the reference (one thread per supernode, kl_chol.cu:166-223). */
 typedef struct {
   int32_t max_ns[3];    /* increasing, 1 .. 144 */
@@ -209,12 +209,12 @@ typedef enum {
 } mbc_matvec_impl;
 
 /* Choose the matvec implementation of an FP32 point-kernel solver (checks,
- * A/B timing).  Dense operators always use the CUDA-core kernels; FP64
+ * A/B timing).  Dense operators have their own FP32 kernels; FP64
  * matvecs follow mbc_solver_set_fp64_matvec. */
 mbc_status mbc_solver_set_matvec(mbc_solver *s, int32_t impl);
 
 typedef enum {
-  MBC_FP64_MATVEC_SIMT = 0, /* FP64 CUDA-core kernels (the default) */
+  MBC_FP64_MATVEC_SIMT = 0, /* FP64 kernels (the default) */
   MBC_FP64_MATVEC_INT8 = 1  /* FP64-accurate INT8 tensor-core matvec (exact digit slicing) */
 } mbc_fp64_matvec;
 
