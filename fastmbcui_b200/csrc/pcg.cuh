@@ -91,18 +91,6 @@ __device__ __forceinline__ void apply_sum(int32_t mode, int c, double s, const P
     case RED_REPLACE:
       if (sc.status[c] == COL_ACTIVE || sc.status[c] == COL_MAXIT) {
         const double prev = sc.rr_ref[c];
-        // A true residual well above the recursive one (norm ratio over
-        // sqrt 2) does not continue the recursion: the next beta, a ratio
-        // over the recursive r.z, would be huge and leave the stale p in
-        // front of every later direction, hundreds to thousands of
-        // iterations without a step.  Such a column starts over from its
-        // preconditioned residual (beta = 0); others keep p.  Measured:
-        // 9600 points of boxes above a floor, 36 columns to 1e-10, 584
-        // iterations and 17 columns finished in FP64 (545 ms) -> 24 and
-        // none (27 ms); scenes that need hundreds of iterations stay
-        // within a few per cent (starting over at every replacement costs
-        // them up to 60 %).
-        if (s > 2.0 * sc.rr[c]) sc.rz[c] = __longlong_as_double(0x7ff0000000000000LL);
         sc.rr[c] = s;
         sc.rr_ref[c] = s;
         if (!(s == s)) {
