@@ -46,7 +46,7 @@
 // What bounds it: shared memory, ~1700 of the ~2000 cycles of a k-step at 96
 // columns (MMA operand reads 660, producer stores and coordinate loads 770 to
 // 1100, bulk copies 200); the producers issue for 990.  Measured (B200): K and
-// K^T of 64000 x 64000, 96 columns 20.2 -> 14.1 ms against one producer group,
+// K^T of 64000 x 64000, 96 columns 20.2 -> 14.4 ms against one producer group,
 // two A stages, cvt.rna.tf32 and no parts; 9600 outputs, 36 columns 0.38 -> 0.2 ms.
 // Every mbarrier wait is bounded: on expiry the kernel records the failure in
 // *err, stops waiting, releases the waiters it feeds, waits (bounded) for its
@@ -131,16 +131,22 @@ __host__ __device__ __forceinline__ uint32_t sw128(int row, int k)
                     ((k & 3) << 2));
 }
 
-// nearest TF32 value, ties away from zero, in integer arithmetic: half a unit
-// is added to the magnitude and the 13 low bits dropped.  (cvt.rna.tf32 does
-// the same at a sixteenth of the rate; two per kernel value were a fifth of
-// the producers' time.)
+// nearest TF32 value of a finite or infinite v, ties away from zero, in integer
+// arithmetic: half a unit is added to the magnitude and the 13 low bits
+// dropped.  (cvt.rna.tf32 does the same at a sixteenth of the rate; two per
+// kernel value were a fifth of the producers' time.)  A NaN does not survive:
+// 0x7fffffff, the one that arithmetic returns, carries into the sign and
+// becomes -0.
 __device__ __forceinline__ uint32_t tf32_rna(float v) { return (__float_as_uint(v) + 0x1000u) & 0xffffe000u; }
 
+// v = hi + lo to 22 bits.  The remainder of a NaN or infinite v is NaN whatever
+// hi has become, and lo is then a NaN in TF32 too, so that it reaches the
+// products (two instructions of the producers' ~30 per value; cvt.rna kept it).
 __device__ __forceinline__ void split_tf32(float v, uint32_t &hi, uint32_t &lo)
 {
   hi = tf32_rna(v);
-  lo = tf32_rna(v - __uint_as_float(hi));
+  const float d = v - __uint_as_float(hi);
+  lo = d == d ? tf32_rna(d) : 0x7fc00000u;
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
