@@ -69,7 +69,10 @@ __global__ void __launch_bounds__(128) solid_angle_kernel(int n_vert, const floa
 //     FP32 estimate after one Newton step (1e-14), kept in shared memory;
 //   * has R1 . (R2 x R3) = R1 . n with the face's n = (v2 - v1) x (v3 - v1), and
 //     Ri . Rj = (qi + qj - |vi - vj|^2) / 2, so that an entry divided by
-//     l1 l2 l3 is num = (R1 . n) y1 y2 y3 over den = 1 + sum (Ri . Rj) yi yj;
+//     l1 l2 l3 is num = (R1 . n) y1 y2 y3 over den = 1 + sum (Ri . Rj) yi yj.
+//     Only differences of a face's own vertices and a source enter an entry: a
+//     vertex that is NaN, infinite or far from the others changes the faces
+//     that name it and no others of its tile;
 //   * for |num| <= den / 4 (all but the few sources next to a face) takes
 //     atan(num / den) from its Maclaurin series, 4 terms below 0.02 and 10 up to
 //     0.25 (errors 3e-15 and 5e-14 of the value); the other entries take the
@@ -77,7 +80,7 @@ __global__ void __launch_bounds__(128) solid_angle_kernel(int n_vert, const floa
 //     leave FP32's range and faces without a vertex (NaN).
 // About 40 FP64 instructions an entry instead of 190; the error is the FP32
 // rounding of the stored value, as before.  Measured (B200, 30720 x 15372):
-// 4.90 -> 2.38 ms; the FP64 pipe is 45 % busy, the rest waits for the chains of
+// 4.90 -> 2.42 ms; the FP64 pipe is 45 % busy, the rest waits for the chains of
 // FP64 results (16 warps per SM).  FP64 matrices keep the kernel
 // above.
 constexpr int kFT = 16, kST = 128, kMaxV = 3 * kFT, kAsmThreads = 256;
@@ -122,8 +125,8 @@ __global__ void __launch_bounds__(kAsmThreads, 2) solid_angle_f32_kernel(int n_v
   extern __shared__ double dyn[];
   double *vq = dyn, *vy = dyn + kMaxV * kST;  // [vertex][source]
   __shared__ int s_id[kMaxV], s_first[kMaxV], s_slot[kMaxV], s_nu;
-  __shared__ double s_v[3][kMaxV];   // distinct vertices, relative to the block's origin
-  __shared__ __align__(16) double s_f[kFT][8];  // n, v1 . n, half the squared edges of a face
+  __shared__ double s_v[3][kMaxV];   // distinct vertices
+  __shared__ __align__(16) double s_f[kFT][10];  // n, v1, half the squared edges of a face
   __shared__ __align__(16) int4 s_c[kFT];       // its corners' slots, times kST
   const int tid = threadIdx.x;
   const int j = tid & (kST / 2 - 1), fg = tid / (kST / 2);  // sources j and j + kST / 2
@@ -136,8 +139,6 @@ __global__ void __launch_bounds__(kAsmThreads, 2) solid_angle_f32_kernel(int n_v
       s_id[tid] = v >= 0 && v < n_vert ? v : -1;
     }
     __syncthreads();
-    const int org = max(s_id[0], 0);
-    const double ox = V[3 * (size_t)org], oy = V[3 * (size_t)org + 1], oz = V[3 * (size_t)org + 2];
     if (tid < kMaxV) {
       int k = 0;
       while (s_id[k] != s_id[tid]) ++k;
@@ -150,9 +151,8 @@ __global__ void __launch_bounds__(kAsmThreads, 2) solid_angle_f32_kernel(int n_v
       s_slot[tid] = slot;
       if (s_first[tid] == tid) {
         const int v = s_id[tid];
-        s_v[0][slot] = v < 0 ? nan("") : V[3 * (size_t)v] - ox;
-        s_v[1][slot] = v < 0 ? nan("") : V[3 * (size_t)v + 1] - oy;
-        s_v[2][slot] = v < 0 ? nan("") : V[3 * (size_t)v + 2] - oz;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) s_v[d][slot] = v < 0 ? nan("") : V[3 * (size_t)v + d];
       }
       if (tid == kMaxV - 1) {
         int nu = 0;
@@ -180,10 +180,11 @@ __global__ void __launch_bounds__(kAsmThreads, 2) solid_angle_f32_kernel(int n_v
       s_f[tid][0] = n0;
       s_f[tid][1] = n1;
       s_f[tid][2] = n2;
-      s_f[tid][3] = v[0][0] * n0 + v[0][1] * n1 + v[0][2] * n2;
-      s_f[tid][4] = 0.5 * (e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2]);
-      s_f[tid][5] = 0.5 * (e2[0] * e2[0] + e2[1] * e2[1] + e2[2] * e2[2]);
-      s_f[tid][6] = 0.5 * (e3[0] * e3[0] + e3[1] * e3[1] + e3[2] * e3[2]);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) s_f[tid][3 + d] = v[0][d];
+      s_f[tid][6] = 0.5 * (e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2]);
+      s_f[tid][7] = 0.5 * (e2[0] * e2[0] + e2[1] * e2[1] + e2[2] * e2[2]);
+      s_f[tid][8] = 0.5 * (e3[0] * e3[0] + e3[1] * e3[1] + e3[2] * e3[2]);
     }
     const int nu = s_nu;
     for (int tl = 0; tl < tiles_per; ++tl) {
@@ -193,9 +194,9 @@ __global__ void __launch_bounds__(kAsmThreads, 2) solid_angle_f32_kernel(int n_v
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int js = min(j0 + j + h * (kST / 2), n_src - 1);
-        sx[h] = S[3 * (size_t)js] - ox;
-        sy[h] = S[3 * (size_t)js + 1] - oy;
-        sz[h] = S[3 * (size_t)js + 2] - oz;
+        sx[h] = S[3 * (size_t)js];
+        sy[h] = S[3 * (size_t)js + 1];
+        sz[h] = S[3 * (size_t)js + 2];
       }
       __syncthreads();  // the face constants, or the last tile's readers
       for (int u = fg; u < nu; u += kFG) {
@@ -215,9 +216,10 @@ __global__ void __launch_bounds__(kAsmThreads, 2) solid_angle_f32_kernel(int n_v
       for (int f = fg; f < nfc; f += kFG, row += kFG * ldm) {
         const int4 c = s_c[f];
         const double2 n01 = *reinterpret_cast<const double2 *>(&s_f[f][0]);
-        const double2 n2h = *reinterpret_cast<const double2 *>(&s_f[f][2]);
-        const double2 c01 = *reinterpret_cast<const double2 *>(&s_f[f][4]);
-        const double c2 = s_f[f][6];
+        const double2 n2v = *reinterpret_cast<const double2 *>(&s_f[f][2]);
+        const double2 v12 = *reinterpret_cast<const double2 *>(&s_f[f][4]);
+        const double2 c01 = *reinterpret_cast<const double2 *>(&s_f[f][6]);
+        const double c2 = s_f[f][8];
         double num[2], t[2];
         bool fine[2];
 #pragma unroll
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(kAsmThreads, 2) solid_angle_f32_kernel(int n_v
           const double p12 = y1 * y2, p = p12 * y3;
           const double d12 = fma(0.5, q1 + q2, -c01.x), d13 = fma(0.5, q1 + q3, -c01.y), d23 = fma(0.5, q2 + q3, -c2);
           const double den = fma(d12, p12, fma(d13, y1 * y3, fma(d23, y2 * y3, 1.0)));
-          num[h] = fma(-sx[h], n01.x, fma(-sy[h], n01.y, fma(-sz[h], n2h.x, n2h.y))) * p;
+          num[h] = fma(n2v.y - sx[h], n01.x, fma(v12.x - sy[h], n01.y, (v12.y - sz[h]) * n2v.x)) * p;
           const double r0 = (double)__fdividef(1.0f, (float)den);
           t[h] = num[h] * fma(r0, fma(-den, r0, 1.0), r0);
           fine[h] = fabs(num[h]) <= 0.25 * den && p > 1e-50 && p < 1e50;
