@@ -73,19 +73,30 @@ __global__ void __launch_bounds__(128) solid_angle_kernel(int n_vert, const floa
 //     Only differences of a face's own vertices and a source enter an entry: a
 //     vertex that is NaN, infinite or far from the others changes the faces
 //     that name it and no others of its tile;
-//   * for |num| <= den / 4 (all but the few sources next to a face) takes
-//     atan(num / den) from its Maclaurin series, 4 terms below 0.02 and 10 up to
-//     0.25 (errors 3e-15 and 5e-14 of the value); the other entries take the
-//     formula with square roots and atan2, as do coordinates whose squares
-//     leave FP32's range and faces without a vertex (NaN).
+//   * for |num| <= (den - 0.01) / 4 (all but the few sources next to a face or
+//     its edges) takes atan(num / den) from its Maclaurin series, 4 terms below
+//     0.02 and 10 up to 0.25 (errors 3e-15 and 5e-14 of the value); the other
+//     entries take the formula with square roots and atan2.  So do those
+//     where the form above cancels: den by its absolute error of ~3e-13 (y) and
+//     ~3e-16 times the ratio of the longest to the shortest of l1, l2, l3, R1 . n
+//     by that ratio too.  With den at least 0.01 and the ratio at most 256 an
+//     entry keeps 1e-10, a thousandth of the FP32 rounding.  And so do distances outside 1e-17 .. 1e17, whose squares
+//     leave FP32's range, and faces without a vertex (NaN);
 // About 40 FP64 instructions an entry instead of 190; the error is the FP32
 // rounding of the stored value, as before.  Measured (B200, 30720 x 15372):
-// 4.90 -> 2.42 ms; the FP64 pipe is 45 % busy, the rest waits for the chains of
+// 4.90 -> 2.49 ms; the FP64 pipe is 40 to 45 % busy, the rest waits for the chains of
 // FP64 results (16 warps per SM).  FP64 matrices keep the kernel
 // above.
 constexpr int kFT = 16, kST = 128, kMaxV = 3 * kFT, kAsmThreads = 256;
 constexpr int kFG = kAsmThreads / (kST / 2);  // groups of faces; a thread takes two sources
 constexpr int kAsmSmem = 2 * kMaxV * kST * (int)sizeof(double);
+
+constexpr double kMinDen = 0.01;
+// upper words of positive doubles order as integers: the smallest y = 1 / l in
+// 1e-17 .. 1e17 / 2^8 (a NaN's word lies outside), the largest within a factor
+// of 2^8 of it
+constexpr int kYLow = 0x3c670ef5;
+constexpr unsigned kYRatio = 8u << 20, kYSpan = 0x43763457u - kYLow - kYRatio;
 
 // atan(t), |t| <= 1/4, from its Maclaurin series
 __device__ __forceinline__ double atan_quarter(double t)
@@ -233,7 +244,10 @@ __global__ void __launch_bounds__(kAsmThreads, 2) solid_angle_f32_kernel(int n_v
           num[h] = fma(n2v.y - sx[h], n01.x, fma(v12.x - sy[h], n01.y, (v12.y - sz[h]) * n2v.x)) * p;
           const double r0 = (double)__fdividef(1.0f, (float)den);
           t[h] = num[h] * fma(r0, fma(-den, r0, 1.0), r0);
-          fine[h] = fabs(num[h]) <= 0.25 * den && p > 1e-50 && p < 1e50;
+          const int e1 = __double2hiint(y1), e2 = __double2hiint(y2), e3 = __double2hiint(y3);
+          const int ya = min(e1, min(e2, e3)), yb = max(e1, max(e2, e3));
+          fine[h] = fabs(num[h]) <= fma(0.25, den, -0.25 * kMinDen) && (unsigned)(ya - kYLow) <= kYSpan &&
+                    (unsigned)(yb - ya) <= kYRatio;
         }
         double out[2];
         if (__all_sync(0xffffffffu, fine[0] && fine[1] && fabs(t[0]) < 0.02 && fabs(t[1]) < 0.02)) {
