@@ -290,7 +290,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 || NT <= 2 ? 2 : 1) d
   __syncthreads();
 
   // the block's sum: warps 4..7 hand theirs to warps 0..3, whose four blocks
-  // are then added in order.  slot[w][output][column]
+  // are then added in order (there and over the cluster in 64 bits, with one
+  // rounding each, as every rounding of a whole sum weighs as much as a
+  // warp's chain).  slot[w][output][column]
   T *slot = reinterpret_cast<T *>(smd);
   constexpr int SL = kBM * NP;
   auto visit = [&](auto f) {  // f(element of the 64 x NP block, accumulator index)
@@ -317,7 +319,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 || NT <= 2 ? 2 : 1) d
   if (warp < 4) visit([&](int e, int q) { mine[e] += acc[q]; });
   __syncthreads();
   T *fin = slot + 4 * SL;
-  for (int e = tid; e < SL; e += kThreads) fin[e] = (slot[e] + slot[SL + e]) + (slot[2 * SL + e] + slot[3 * SL + e]);
+  for (int e = tid; e < SL; e += kThreads)
+    fin[e] = (T)(((double)slot[e] + (double)slot[SL + e]) + ((double)slot[2 * SL + e] + (double)slot[3 * SL + e]));
 
   // the cluster's blocks hold the shares of the reduction axis: each adds and
   // stores a slice of the outputs
@@ -341,8 +344,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 || NT <= 2 ? 2 : 1) d
       T s;
       if (z > 1) {
         cg::cluster_group cl = cg::this_cluster();
-        s = *cl.map_shared_rank(fin + o * NP + c, 0);
-        for (int k = 1; k < z; ++k) s += *cl.map_shared_rank(fin + o * NP + c, k);
+        double sum = *cl.map_shared_rank(fin + o * NP + c, 0);
+        for (int k = 1; k < z; ++k) sum += (double)*cl.map_shared_rank(fin + o * NP + c, k);
+        s = (T)sum;
       } else {
         s = fin[o * NP + c];
       }
