@@ -4,6 +4,7 @@
 #include <atomic>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -107,8 +108,12 @@ void DevMem::release()
       cudaFree(ptr);
     } else {
       trim(p, p.bound - size_);
-      p.idle.emplace(size_, Pool::Block{ptr, ++p.seq});
-      p.idle_bytes += size_;
+      try {
+        p.idle.emplace(size_, Pool::Block{ptr, ++p.seq});
+        p.idle_bytes += size_;
+      } catch (const std::bad_alloc &) {  // a destructor may be the caller
+        cudaFree(ptr);
+      }
     }
   }
   ptr = nullptr;
@@ -201,6 +206,11 @@ int32_t *pinned_flags()
 {
   std::lock_guard<std::mutex> lk(g_flag_mu);
   if (!g_flag_page) {
+    try {
+      g_flag_free.reserve(kSlots);  // no later push allocates
+    } catch (const std::bad_alloc &) {
+      return nullptr;
+    }
     if (cudaHostAlloc((void **)&g_flag_page, sizeof(int32_t) * 4 * kSlots, cudaHostAllocPortable) != cudaSuccess) {
       cudaGetLastError();
       g_flag_page = nullptr;
