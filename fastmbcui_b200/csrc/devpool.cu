@@ -128,35 +128,33 @@ mbc_status DevMem::reserve(size_t b)
   if (b == 0) b = 16;
   int dev = -1;
   MBC_CK(cudaGetDevice(&dev));
-  cudaError_t e = cudaSuccess;
-  if (pooled_ && dev >= 0 && dev < kMaxDevices) {
-    Pool &p = g_pools[dev];
-    std::lock_guard<std::mutex> lk(p.mu);
-    if (p.bound == 0) {
+  Pool *p = dev >= 0 && dev < kMaxDevices ? &g_pools[dev] : nullptr;
+  std::unique_lock<std::mutex> lk;
+  if (p) lk = std::unique_lock<std::mutex>(p->mu);
+  dev_ = -1;
+  size_ = b;
+  if (pooled_ && p) {
+    if (p->bound == 0) {
       size_t free_b = 0, total_b = 0;
       MBC_CK(cudaMemGetInfo(&free_b, &total_b));
-      p.bound = std::min<size_t>(kBound, total_b / 16);
-    }
-    size_ = rounded(b);
-    auto it = p.idle.lower_bound(size_);
-    if (it != p.idle.end() && it->first <= size_ + size_ / 8) {
-      ptr = it->second.ptr;
-      size_ = it->first;
-      p.idle_bytes -= it->first;
-      p.idle.erase(it);
-    } else {
-      e = cudaMalloc(&ptr, size_);
-      if (e == cudaErrorMemoryAllocation && !p.idle.empty()) {
-        cudaGetLastError();
-        trim(p, 0);
-        e = cudaMalloc(&ptr, size_);
-      }
+      p->bound = std::min<size_t>(kBound, total_b / 16);
     }
     dev_ = dev;
-  } else {
-    size_ = b;
-    e = cudaMalloc(&ptr, b);
-    dev_ = -1;
+    size_ = rounded(b);
+    auto it = p->idle.lower_bound(size_);
+    if (it != p->idle.end() && it->first <= size_ + size_ / 8) {
+      ptr = it->second.ptr;
+      size_ = it->first;
+      p->idle_bytes -= it->first;
+      p->idle.erase(it);
+    }
+  }
+  cudaError_t e = ptr ? cudaSuccess : cudaMalloc(&ptr, size_);
+  if (e == cudaErrorMemoryAllocation && p && !p->idle.empty()) {
+    // the pool's idle memory goes before any allocation of the library fails
+    cudaGetLastError();
+    trim(*p, 0);
+    e = cudaMalloc(&ptr, size_);
   }
   if (e != cudaSuccess) {
     ptr = nullptr;

@@ -182,6 +182,20 @@ void trim()
   CHECK(more.reserve(kGiB) == MBC_OK);
 }
 
+// ... also one that does not come from the pool itself
+void trim_unpooled()
+{
+  mbc::PoolUser user;
+  {
+    DevMem a;
+    CHECK(a.reserve(3 * kGiB) == MBC_OK);
+  }
+  DevMem big(false);
+  CHECK(big.reserve(63 * kGiB) == MBC_OK && g_live.size() == 1);
+  big.release();
+  CHECK(g_live.empty());
+}
+
 // inside a call a release waits for the call's stream, a failing call for its
 // work; outside of calls nothing waits
 void waits()
@@ -228,7 +242,7 @@ void host_memory()
 int main(int argc, char **argv)
 {
   const std::map<std::string, void (*)()> checks = {
-      {"reuse", reuse}, {"bound", bound}, {"trim", trim}, {"waits", waits}, {"host_memory", host_memory}};
+      {"reuse", reuse}, {"bound", bound}, {"trim", trim}, {"trim_unpooled", trim_unpooled}, {"waits", waits}, {"host_memory", host_memory}};
   auto it = checks.find(argc > 1 ? argv[1] : "");
   if (it == checks.end()) return 2;
   it->second();
