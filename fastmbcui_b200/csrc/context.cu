@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include "mbc_internal.h"
+#include "solver.h"
 
 using mbc::fail;
 
@@ -40,6 +41,7 @@ extern "C" mbc_status mbc_context_create(mbc_context **out)
 
 extern "C" mbc_status mbc_context_destroy(mbc_context *ctx)
 {
+  mbc::PoolUser hold;  // the last one to go, if no other object is alive
   delete ctx;
   return MBC_OK;
 }
@@ -125,6 +127,15 @@ mbc_status run(mbc_context *ctx, bool adjoint, const float *M, int32_t nf, int32
   if (adjoint && !ctx->has_forward)
     return fail(MBC_BAD_ARG, "Float cache tensors are not defined. Please run MinvF_float first.");
   if (maxit < 0 || maxit > (int64_t)1 << 30) return fail(MBC_BAD_ARG, "pcg_max_iter out of range");
+  struct Hold {  // the pool has a user during the call; the kept plan and solver are none after it
+    mbc_context *ctx;
+    mbc::PoolUser user;
+    ~Hold()
+    {
+      if (ctx->plan) ctx->plan->user.leave();
+      if (ctx->solver) ctx->solver->user.leave();
+    }
+  } hold{ctx, {}};
   auto t0 = clk::now();
   bool reused = false;
   s = prepare(ctx, M, nf, n, Vs_host, rho, adjoint, timing != 0, st, &reused);

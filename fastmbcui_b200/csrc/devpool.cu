@@ -2,6 +2,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <map>
 #include <mutex>
 #include <new>
@@ -16,6 +17,11 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 constexpr size_t kBound = (size_t)8 << 30;  // idle bytes a pool keeps: at most this and a sixteenth of the device
+// ... while a quarter of the device is free besides (others, such as a tensor
+// library's allocator, come first), looked at as a plan or solver ends, but not
+// again within this time: the question takes the driver 0.1 ms and more
+constexpr size_t kRoom = 4;
+constexpr std::chrono::milliseconds kLook(200);
 
 // Idle cudaMalloc blocks of one device, by size.  (The driver's own
 // stream-ordered pools hand out kept memory as fast, but take 5 ms per GB to
@@ -28,6 +34,7 @@ struct Pool {
   };
   std::multimap<size_t, Block> idle;
   size_t idle_bytes = 0, bound = 0;
+  std::chrono::steady_clock::time_point looked{};  // at the device's free memory
   uint64_t seq = 0;
 };
 Pool g_pools[kMaxDevices];
@@ -181,11 +188,18 @@ void pool_retain() { ++g_alive; }
 
 void pool_drop()
 {
-  if (--g_alive != 0) return;
+  const bool last = --g_alive == 0;
   for (int d = 0; d < kMaxDevices; ++d) {
     std::lock_guard<std::mutex> lk(g_pools[d].mu);
     if (g_pools[d].idle.empty()) continue;
     DeviceGuard on(d);
+    if (!last) {
+      const auto now = std::chrono::steady_clock::now();
+      size_t free_b = 0, total_b = 0;
+      if (now - g_pools[d].looked < kLook) continue;
+      g_pools[d].looked = now;
+      if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b >= total_b / kRoom) continue;
+    }
     trim(g_pools[d], 0);
   }
 }

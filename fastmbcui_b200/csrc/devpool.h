@@ -36,9 +36,10 @@ class CallScope {
 
 // Owned device allocation that only grows; memory of the current device's
 // pool.  The pool keeps what is released, at most 8 GiB and a sixteenth of the
-// device, for the next solver of any thread and stream, gives it back when an
-// allocation of this library would fail, and all of it once no plan and no
-// solver is alive.
+// device, for the next solver of any thread and stream.  It gives all of it
+// back when an allocation of this library would fail, when a plan or solver
+// ends on a device with less than a quarter free, and once no plan and no
+// solver is alive but those that an operator context keeps between its calls.
 struct DevMem {
   void *ptr = nullptr;
   size_t bytes = 0;

@@ -45,14 +45,24 @@ mbc_status build_supernodes(Plan &p, int n_threads);
 mbc_status spatial_order(int32_t n, const float *pts, int32_t stride, int32_t *order);
 
 // Plans and solvers alive: the last one to go empties the device memory pools
-// (devpool.h).
+// (devpool.h).  One that a context keeps for its next call doesn't count
+// between calls (leave), so that a program which called an operator once does
+// not hold idle memory for good.
 void pool_retain();
 void pool_drop();
 struct PoolUser {
   PoolUser() { pool_retain(); }
-  ~PoolUser() { pool_drop(); }
+  ~PoolUser() { leave(); }
   PoolUser(const PoolUser &) = delete;
   PoolUser &operator=(const PoolUser &) = delete;
+  void leave()
+  {
+    if (counted_) pool_drop();
+    counted_ = false;
+  }
+
+ private:
+  bool counted_ = true;
 };
 
 }  // namespace mbc

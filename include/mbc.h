@@ -17,8 +17,10 @@
  *   - mbc_stream is cudaStream_t; NULL is the legacy default stream.
  *   - Objects are caller-owned.  Between solvers the library keeps idle device
  *     memory in a pool (per device at most 8 GiB and a sixteenth of it), returned
- *     when an allocation of its own would fail and when the last plan and
- *     solver are destroyed; nothing else outlives the objects.
+ *     when an allocation of its own would fail, when a plan or solver is
+ *     destroyed on a device with less than a quarter free, and when the last
+ *     plan and solver are destroyed (those inside an mbc_context count only
+ *     during its calls); nothing else outlives the objects.
  */
 #ifndef MBC_H
 #define MBC_H

@@ -1,6 +1,7 @@
 // The device memory pool (devpool.cu, compiled as host code) against a fake
 // CUDA runtime: two devices of a given size, allocations counted, streams
 // that record when they are waited for.  Run with the name of one check.
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -196,6 +197,47 @@ void trim_unpooled()
   CHECK(g_live.empty());
 }
 
+// what a kept object holds between its calls is no reason to keep idle memory
+void leave()
+{
+  mbc::PoolUser *kept = new mbc::PoolUser();
+  DevMem own;
+  {
+    mbc::PoolUser call;
+    DevMem a;
+    CHECK(own.reserve(MiB) == MBC_OK && a.reserve(kGiB) == MBC_OK);
+    a.release();
+    CHECK(g_live.size() == 2);
+    kept->leave();
+    CHECK(g_live.size() == 2);
+  }
+  CHECK(g_live.size() == 1 && own.ptr);
+  {
+    mbc::PoolUser end;
+    own.release();
+    delete kept;  // counted once
+    CHECK(g_live.size() == 1);
+  }
+  CHECK(g_live.empty());
+}
+
+// with less than a quarter of the device free nothing idle outlives a solver
+void room()
+{
+  mbc::PoolUser user;
+  for (size_t others : {40 * kGiB, 50 * kGiB}) {
+    std::this_thread::sleep_for(std::chrono::milliseconds(250));  // it is looked at five times a second
+    g_other[0] = others;
+    {
+      mbc::PoolUser solver;
+      DevMem a;
+      CHECK(a.reserve(2 * kGiB) == MBC_OK);
+    }
+    CHECK(used(0) == others + (others == 40 * kGiB ? 2 * kGiB : 0));
+  }
+  CHECK(t_dev == 0);
+}
+
 // inside a call a release waits for the call's stream, a failing call for its
 // work; outside of calls nothing waits
 void waits()
@@ -242,7 +284,8 @@ void host_memory()
 int main(int argc, char **argv)
 {
   const std::map<std::string, void (*)()> checks = {
-      {"reuse", reuse}, {"bound", bound}, {"trim", trim}, {"trim_unpooled", trim_unpooled}, {"waits", waits}, {"host_memory", host_memory}};
+      {"reuse", reuse}, {"bound", bound}, {"trim", trim}, {"trim_unpooled", trim_unpooled}, {"leave", leave},
+      {"room", room}, {"waits", waits}, {"host_memory", host_memory}};
   auto it = checks.find(argc > 1 ? argv[1] : "");
   if (it == checks.end()) return 2;
   it->second();

@@ -26,7 +26,8 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("check", ["reuse", "bound", "trim", "trim_unpooled", "waits", "host_memory"])
+@pytest.mark.parametrize("check", ["reuse", "bound", "trim", "trim_unpooled", "leave", "room", "waits",
+                                   "host_memory"])
 def test_pool(exe, check):
     r = subprocess.run([exe, check], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stderr)

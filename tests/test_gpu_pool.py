@@ -1,0 +1,43 @@
+"""The operators keep a plan and a solver for the backward pass, but no idle
+device memory after their calls: what an earlier, larger call had is back with
+the device.  In a process of its own, where no other solver is alive.
+
+The larger scene's solver has over 60 MB; the device's free memory after a small
+call may fall short of that before the larger one by 32 MB (the kernels' code, the
+small solver, allocation granularity)."""
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+PROG = """
+import numpy as np, torch
+from fastmbcui_b200.mfs_torch import ops
+
+def call(nf, n):
+    rng = np.random.default_rng(n)
+    k = np.arange(n) + 0.5
+    z, phi = 1.0 - 2.0 * k / n, np.pi * (1.0 + 5.0 ** 0.5) * k
+    y = np.stack([np.sqrt(1 - z * z) * np.cos(phi), np.sqrt(1 - z * z) * np.sin(phi), z], 1).astype(np.float32)
+    M = torch.as_tensor(rng.standard_normal((nf, n)).astype(np.float32), device="cuda")
+    F = torch.as_tensor(rng.standard_normal((nf, 6)).astype(np.float32), device="cuda")
+    ops.MinvF_float_fastGrad(M, F, torch.as_tensor(y), 6.0, 40, 1e-3)
+    del M, F
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+small = call(400, 200)
+large = call(6000, 5000)
+again = call(400, 200)
+assert small - large > 60e6, (small, large)
+assert small - again < 32e6, (small, large, again)
+print("ok")
+"""
+
+
+def test_operator_calls_keep_no_idle_memory():
+    r = subprocess.run([sys.executable, "-c", PROG], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), (r.stdout, r.stderr[-2000:])
