@@ -41,10 +41,11 @@ struct FactorArgs {
   // retry (FP32 launches); 0 flags only non-positive pivots.
   double pivot_tol;
   // 1: Theta_s of every supernode of the launch is already in global memory
-  // (gram_kernel, gram_tc_kernel): step 1 only loads it, the sum in order of
-  // gram_parts copies gram_stride entries apart
+  // (gram_kernel, gram_tc_kernel), at gram_src + gram_off[s]: step 1 only loads
+  // it, the sum in order of gram_parts copies gram_stride entries apart
   int32_t gram_ready;
   const void *gram_src;
+  const int64_t *gram_off;
   int32_t gram_parts;
   int64_t gram_stride;
   int32_t smem_cap;  // largest n_s kept in shared memory
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(NT) factor_kernel(FactorArgs a, T *__restrict_
   // 1. Gram assembly, entry chunks of NT*EPT upper-triangle entries (or,
   // with gram_ready, the sum of the parts in global memory)
   if (a.gram_ready && in_smem) {
-    const T *src = reinterpret_cast<const T *>(a.gram_src) + a.th_ptr[s];
+    const T *src = reinterpret_cast<const T *>(a.gram_src) + a.gram_off[s];
     for (int e = tid; e < ns * ns; e += NT) {
       T v = src[e];
       for (int q = 1; q < a.gram_parts; ++q) v += src[(size_t)q * a.gram_stride + e];

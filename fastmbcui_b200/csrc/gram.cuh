@@ -63,6 +63,7 @@ struct Args {
   FactorArgs f;
   int parts;           // parts of the rows: grid.y
   int64_t part_stride; // entries between the parts' copies of theta
+  const int64_t *off;  // a supernode's entries in a copy
   int rows, ld;        // panel rows and stride of the launch
 };
 
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 || MT <= 2 ? 2 : 1) g
         for (int h = 0; h < cnt; ++h) fin[i] += slot[(size_t)h * W * W + e];
     }
   }
-  T *A = theta + a.part_stride * blockIdx.y + f.th_ptr[s];
+  T *A = theta + a.part_stride * blockIdx.y + a.off[s];
 #pragma unroll
   for (int i = 0; i < kMaxNs * kMaxNs / kThreads; ++i) {
     const int e = tid + i * kThreads, p = e / W, q = e % W;

@@ -371,26 +371,40 @@ static FactorArgs factor_args(const Solver &S)
 
 // Theta of supernodes with at most gram::kMaxNs entries by gram_kernel: one
 // launch per kernel shape.  The rows are cut into as many parts as give about
-// four blocks per SM (at least four panels each, at most half a GB of copies);
-// *src, *parts and *stride are where factor_kernel finds the copies.
+// four blocks per SM (at least four panels each, at most half a GB of copies of
+// the listed sets' Theta; none where there is no memory for them); `g` is where
+// factor_kernel finds them.
+struct GramParts {
+  const void *src = nullptr;
+  int parts = 1;
+  int64_t stride = 0;
+  const int64_t *off = nullptr;  // per supernode
+};
 template <typename T>
-static mbc_status launch_grams(Solver &S, const std::vector<int32_t> &ids, T *theta, const void **src, int *parts,
-                               int64_t *stride, cudaStream_t st)
+static mbc_status launch_grams(Solver &S, const std::vector<int32_t> &ids, T *theta, GramParts &g, cudaStream_t st)
 {
   const Plan &p = *S.plan;
-  const int64_t th_n = p.th_ptr.back();
+  int64_t len = 0;
+  std::vector<int64_t> off(p.n_super, 0);
+  for (int32_t s : ids) {
+    off[s] = len;
+    len += p.th_ptr[s + 1] - p.th_ptr[s];
+  }
   int64_t np = cdiv(4 * 148, (int64_t)ids.size());
   np = std::min<int64_t>(np, std::max(1, S.nf / 512));
-  np = std::min<int64_t>(np, ((int64_t)512 << 20) / std::max<int64_t>(1, th_n * (int64_t)sizeof(T)));
+  np = std::min<int64_t>(np, ((int64_t)512 << 20) / std::max<int64_t>(1, len * (int64_t)sizeof(T)));
   np = std::max<int64_t>(1, std::min<int64_t>(np, gram::kMaxParts));
+  if (np > 1 && S.gram_part.reserve((size_t)np * len * sizeof(T)) != MBC_OK) np = 1;
   T *dst = theta;
+  g.off = S.d_th_ptr();
   if (np > 1) {
-    MBC_TRY(S.gram_part.reserve((size_t)np * th_n * sizeof(T)));
+    MBC_TRY(upload(S.gram_off, off, st));
     dst = (T *)S.gram_part.ptr;
+    g.off = (const int64_t *)S.gram_off.ptr;
   }
-  *src = dst;
-  *parts = (int)np;
-  *stride = th_n;
+  g.src = dst;
+  g.parts = (int)np;
+  g.stride = len;
   // shapes: FP32 up to 32 and 64 entries, FP64 one per 16
   constexpr int kShapes = sizeof(T) == 4 ? 2 : 4, kStep = gram::kMaxNs / kShapes;
   std::vector<int32_t> by[kShapes], all;
@@ -412,7 +426,8 @@ static mbc_status launch_grams(Solver &S, const std::vector<int32_t> &ids, T *th
     a.f.list = (const int32_t *)S.gram_ids.ptr + at;
     a.f.count = (int32_t)by[k].size();
     a.parts = (int)np;
-    a.part_stride = th_n;
+    a.part_stride = g.stride;
+    a.off = g.off;
     a.rows = gram::rows_for<T>(ns_max);
     a.ld = gram::ld_for<T>(ns_max);
     const int smem = gram::smem_bytes<T>(ns_max);
@@ -466,10 +481,8 @@ static mbc_status run_factor(Solver &S, const std::vector<int32_t> *lists, T *th
     }
   if constexpr (std::is_same<T, float>::value)
     if (!gram.empty()) MBC_TRY(launch_gram(S, gram, theta, st));
-  const void *gram_src = nullptr;
-  int gram_parts = 1;
-  int64_t gram_stride = 0;
-  if (!small.empty()) MBC_TRY(launch_grams<T>(S, small, theta, &gram_src, &gram_parts, &gram_stride, st));
+  GramParts g;
+  if (!small.empty()) MBC_TRY(launch_grams<T>(S, small, theta, g, st));
   for (int job = 0; job < 12; ++job) {
     const int c = job & 3, from = job >> 2;  // Theta: 0 factor_kernel's own, 1 tensor cores, 2 gram_kernel
     const auto &lst = from == 0 ? simt[c] : from == 1 ? tcl[c] : grl[c];
@@ -484,9 +497,10 @@ static mbc_status run_factor(Solver &S, const std::vector<int32_t> *lists, T *th
     a.shift = shift;
     a.pivot_tol = pivot_tol;
     a.gram_ready = from != 0;
-    a.gram_src = from == 2 ? gram_src : theta;
-    a.gram_parts = from == 2 ? gram_parts : 1;
-    a.gram_stride = gram_stride;
+    a.gram_src = from == 2 ? g.src : theta;
+    a.gram_off = from == 2 ? g.off : a.th_ptr;
+    a.gram_parts = from == 2 ? g.parts : 1;
+    a.gram_stride = g.stride;
     a.bad_list = d_bad_list;
     a.bad_count = d_bad_count;
     const int nt = kClassThreads[c];
@@ -603,6 +617,7 @@ mbc_status Solver::factor(cudaStream_t st)
     row_values_kernel<float><<<cdiv(l_n, 256), 256, 0, st>>>((int64_t)l_n, d_rmap(), (const float *)lval.ptr, (float *)lrow.ptr);
   MBC_CKL();
   MBC_CK(cudaStreamSynchronize(st));
+  gram_part.release();  // only a factor needs the copies of Theta
   factored = true;
   return MBC_OK;
 }

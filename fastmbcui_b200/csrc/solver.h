@@ -40,7 +40,7 @@ struct Solver {
       m_rmap, m_th_ptr;
   DevMem class_list[4];
   DevMem class_list_tc[4], gram_list;  // FP32 factor: supernodes whose Gram ran on the tensor cores
-  DevMem class_list_gr[4], gram_ids, gram_part;  // supernodes of gram_kernel, its copies of Theta by part
+  DevMem class_list_gr[4], gram_ids, gram_part, gram_off;  // supernodes of gram_kernel, its copies of Theta by part
   int32_t gram_tc_count = 0;           // supernodes of the last factor with the tensor-core Gram
   // operator: rows (original order) and sources (new order) as float4
   DevMem m_x4, m_n4, m_y4;

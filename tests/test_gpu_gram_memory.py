@@ -1,0 +1,40 @@
+"""The FP64 retry of a few supernodes of an FP32 factor takes copies of their
+Theta for the parts of its rows, not of the whole scene's: the device memory that
+factor() takes is that of its results (Theta in FP32 and FP64, L twice), plus
+64 MB of lists, workspaces and granularity.  In a process of its own, where no
+other solver is alive."""
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+PROG = """
+import numpy as np, torch
+import fastmbcui_b200 as F
+
+n, nf = 12000, 8200
+k = np.arange(n) + 0.5
+z, phi = 1.0 - 2.0 * k / n, np.pi * (1.0 + 5.0 ** 0.5) * k
+y = np.stack([np.sqrt(1 - z * z) * np.cos(phi), np.sqrt(1 - z * z) * np.sin(phi), z], 1).astype(np.float32)
+M = torch.randn(nf, n, generator=torch.Generator(device="cuda").manual_seed(0), device="cuda")
+near = int(np.argsort(((y - y[5000]) ** 2).sum(1))[1])
+M[:, near] = M[:, 5000] * 1.00001 + 1e-3 * M[:, near]  # nearly dependent columns: their pivots ask for FP64
+plan = F.Plan(y)
+s = F.Solver(plan, M=M, precision=F.MBC_F32)
+torch.cuda.synchronize()
+before = torch.cuda.mem_get_info()[0]
+s.factor()
+took = before - torch.cuda.mem_get_info()[0]
+assert 1 <= s.pivot_retries() <= 30, s.pivot_retries()
+results = 12 * plan.info.theta_nnz + 8 * plan.info.factor_nnz
+assert 16 * 8 * plan.info.theta_nnz > results + 128e6, plan.info.theta_nnz  # the case can tell
+assert took <= results + 64e6, (took, results)
+print("ok")
+"""
+
+
+def test_retry_of_few_sets_takes_little_memory():
+    r = subprocess.run([sys.executable, "-c", PROG], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), (r.stdout, r.stderr[-2000:])
