@@ -2002,13 +2002,8 @@ extern "C" mbc_status mbc_solver_get_factor_tiles(const mbc_solver *s, mbc_facto
   return MBC_OK;
 }
 
-extern "C" mbc_status mbc_solver_tune_factor(mbc_solver *s, int32_t reps, mbc_factor_tiles *best_out,
-                                             double *ms_best, mbc_stream stream)
+static mbc_status tune_factor(mbc::Solver &S, int32_t reps, mbc_factor_tiles *best_out, double *ms_best, cudaStream_t st)
 {
-  if (!s || reps < 1) return fail(MBC_BAD_ARG, "NULL solver or reps < 1");
-  mbc::Solver &S = s->s;
-  cudaStream_t st = (cudaStream_t)stream;
-  mbc::CallScope scope(st);
   cudaEvent_t e0, e1;
   MBC_CK(cudaEventCreate(&e0));
   MBC_CK(cudaEventCreate(&e1));
@@ -2086,6 +2081,14 @@ extern "C" mbc_status mbc_solver_tune_factor(mbc_solver *s, int32_t reps, mbc_fa
   if (best_out) *best_out = best;
   if (ms_best) *ms_best = tbest;
   return MBC_OK;
+}
+
+extern "C" mbc_status mbc_solver_tune_factor(mbc_solver *s, int32_t reps, mbc_factor_tiles *best_out,
+                                             double *ms_best, mbc_stream stream)
+{
+  if (!s || reps < 1) return fail(MBC_BAD_ARG, "NULL solver or reps < 1");
+  mbc::CallScope scope((cudaStream_t)stream);
+  return scope.end(tune_factor(s->s, reps, best_out, ms_best, (cudaStream_t)stream));
 }
 
 extern "C" mbc_status mbc_solver_set_wait_limit(mbc_solver *s, uint32_t polls)

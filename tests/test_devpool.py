@@ -31,3 +31,20 @@ def exe(tmp_path_factory):
 def test_pool(exe, check):
     r = subprocess.run([exe, check], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stderr)
+
+
+def test_every_call_hands_its_result_through_its_scope():
+    """A call that fails may leave work on its stream; CallScope::end waits for
+    it before the pool hands the call's buffers on."""
+    import re
+
+    seen = 0
+    for f in sorted(os.listdir(CSRC)):
+        if not f.endswith(".cu"):
+            continue
+        src = open(os.path.join(CSRC, f)).read()
+        for body in re.findall(r'^extern "C" .*?^}', src, re.S | re.M):
+            if "CallScope " in body:
+                seen += 1
+                assert "scope.end(" in body, body.split("(")[0]
+    assert seen >= 9
