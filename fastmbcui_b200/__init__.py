@@ -238,6 +238,12 @@ class Solver:
         check(load().mbc_solver_get_pivot_retries(self._h, C.byref(c)), "get_pivot_retries")
         return int(c.value)
 
+    def launches(self) -> int:
+        """Kernels this solver's calls have launched so far."""
+        c = C.c_int64(0)
+        check(load().mbc_solver_get_launches(self._h, C.byref(c)), "get_launches")
+        return int(c.value)
+
     def get_factor(self, theta: bool = False):
         lval = np.empty(max(1, self.plan.info.factor_nnz), np.float64)
         th = np.empty(max(1, self.plan.info.theta_nnz), np.float64) if theta else None

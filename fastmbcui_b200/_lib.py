@@ -96,6 +96,7 @@ SIGNATURES = {
     "mbc_solver_factor": (C.c_int, [_vp, _vp]),
     "mbc_solver_get_factor": (C.c_int, [_vp, _vp, _vp]),
     "mbc_solver_get_pivot_retries": (C.c_int, [_vp, C.POINTER(_i32)]),
+    "mbc_solver_get_launches": (C.c_int, [_vp, C.POINTER(C.c_int64)]),
     "mbc_solver_set_matvec": (C.c_int, [_vp, _i32]),
     "mbc_solver_set_fp64_matvec": (C.c_int, [_vp, _i32]),
     "mbc_solver_prepare": (C.c_int, [_vp, _vp]),

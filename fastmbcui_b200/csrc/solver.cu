@@ -525,6 +525,7 @@ static mbc_status run_factor(Solver &S, const std::vector<int32_t> *lists, T *th
       case 2: MBC_TRY((launch_factor_class<T, LT, 512, 17>(a, theta, lval, smem, st))); break;
       default: MBC_TRY((launch_factor_class<T, LT, 512, 16>(a, theta, lval, smem, st))); break;
     }
+    ++S.launches;
   }
   return MBC_OK;
 }
@@ -615,6 +616,7 @@ mbc_status Solver::factor(cudaStream_t st)
     row_values_kernel<double><<<cdiv(l_n, 256), 256, 0, st>>>((int64_t)l_n, d_rmap(), (const double *)lval.ptr, (double *)lrow.ptr);
   else
     row_values_kernel<float><<<cdiv(l_n, 256), 256, 0, st>>>((int64_t)l_n, d_rmap(), (const float *)lval.ptr, (float *)lrow.ptr);
+  ++launches;
   MBC_CKL();
   MBC_CK(cudaStreamSynchronize(st));
   gram_part.release();  // only a factor needs the copies of Theta
@@ -1200,7 +1202,7 @@ static mbc_status run_block_pcg(Solver &S, int R, PcgWork<double> &w, const LT *
     PcgScalars none{};
     launch_reduce(st, (int)La.grid.x, a, w.part, RED_STORE, none, rr);
     block_check_kernel<<<cdiv(a, 256), 256, 0, st>>>(a, d_act, rr, w.sc);
-    S.launches += 6;
+    S.launches += 5;
     MBC_CKL();
     MBC_CK(cudaMemcpyAsync(status.data(), w.sc.status, sizeof(int32_t) * R, cudaMemcpyDeviceToHost, st));
     MBC_CK(cudaMemcpyAsync(h_small + 1, d_flag, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
@@ -2131,6 +2133,13 @@ extern "C" mbc_status mbc_solver_get_pivot_retries(const mbc_solver *s, int32_t 
 {
   if (!s || !count) return fail(MBC_BAD_ARG, "NULL argument");
   *count = s->s.pivot_retries;
+  return MBC_OK;
+}
+
+extern "C" mbc_status mbc_solver_get_launches(const mbc_solver *s, int64_t *count)
+{
+  if (!s || !count) return fail(MBC_BAD_ARG, "NULL argument");
+  *count = s->s.launches;
   return MBC_OK;
 }
 

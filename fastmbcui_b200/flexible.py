@@ -98,15 +98,11 @@ def solve_flexible(s64, s32, F, tol=1e-8, inner_iters=40, keep=20, max_outer=300
     CUDA-event time of the FP64 applications and of the inner matvecs."""
     import torch
 
-    from . import MBC_FP64_MATVEC_INT8
-
     F = F if F.dim() == 2 else F[:, None]
     F64 = F.double().contiguous()
+    launches64 = s64.launches()
     b = F64 if adjoint else s64.apply_KT(F64)
-    # kernels per FP64 direction: one FP64 kernel, or pack + MMA on the INT8 path
-    per_dir = 2 if getattr(s64, "fp64_matvec", 0) == MBC_FP64_MATVEC_INT8 else 1
-    acc = {"inner": 0, "launches": (per_dir + 1) if not adjoint else 0, "t64": 0.0, "n64": 0, "t32": 0.0,
-           "n32": 0}
+    acc = {"inner": 0, "launches": 0, "t64": 0.0, "n64": 0, "t32": 0.0, "n32": 0}
 
     def apply64(v):
         if profile:
@@ -118,7 +114,6 @@ def solve_flexible(s64, s32, F, tol=1e-8, inner_iters=40, keep=20, max_outer=300
             e1.synchronize()
             acc["t64"] += e0.elapsed_time(e1)
         acc["n64"] += 2
-        acc["launches"] += 2 + 2 * per_dir  # permute, K, K^T, permute
         return out
 
     def inner(rs):
@@ -132,7 +127,7 @@ def solve_flexible(s64, s32, F, tol=1e-8, inner_iters=40, keep=20, max_outer=300
 
     X, info = flexible_cg(apply64, inner, b, tol=tol, keep=keep, max_outer=max_outer,
                           x0=None if X0 is None else X0.double())
-    info.update({"fp32_inner_iterations": acc["inner"], "kernel_launches": acc["launches"],
+    info.update({"fp32_inner_iterations": acc["inner"], "kernel_launches": acc["launches"] + s64.launches() - launches64,
                  "t_matvec64_ms": acc["t64"], "n_matvec64": acc["n64"], "t_matvec32_ms": acc["t32"],
                  "n_matvec32": acc["n32"]})
     return X, info

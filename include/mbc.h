@@ -204,6 +204,10 @@ mbc_status mbc_solver_get_tensor_grams(const mbc_solver *s, int32_t *count);
  * non-positive pivots; FP64 solvers: the diagonal-shift retry). */
 mbc_status mbc_solver_get_pivot_retries(const mbc_solver *s, int32_t *count);
 
+/* Kernels the solver's calls have launched since it was created (mbc_solve_stats
+ * has those of one solve). */
+mbc_status mbc_solver_get_launches(const mbc_solver *s, int64_t *count);
+
 typedef enum {
   MBC_MATVEC_AUTO = 0,   /* tensor cores for FP32 point-kernel matvecs with 8 <= R <= 256 */
   MBC_MATVEC_SIMT = 1,   /* CUDA-core kernels only */
