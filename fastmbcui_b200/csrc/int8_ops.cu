@@ -279,6 +279,8 @@ mbc_status mbc::Solver::ensure_oz(cudaStream_t st, int R)
     const int K = std::max(n, nf);
     MBC_TRY(m_oz_b.reserve(oz::bimg_bytes(K, std::max(R, 1))));
     MBC_TRY(m_oz_bexp.reserve(sizeof(int32_t) * oz::bexp_count(K, std::max(R, 1))));
+    // the check takes the way of the products that follow: parts and their sum
+    if (!oz_slab) m_oz_parts.reserve(oz_parts_bytes(*this, 1));
     MBC_TRY(oz_selfcheck(st));
   }
   const int K = std::max(n, nf);

@@ -66,3 +66,14 @@ def test_counted_launches_are_those_that_ran(prec, impl):
     for opts in ({}, {"schedule": F.MBC_SCHED_BLOCK}, {"fp64_recursion": 1}, {"true_residual": 1}):
         (_, st), ran = _kernels(lambda: s.solve(Fm, max_iters=400, **opts))
         assert st["kernel_launches"] == ran, opts
+
+
+def test_first_use_check_of_the_int8_product_takes_the_split_path():
+    # 3000 points: two parts.  Planes of two directions; the check's INT8 products
+    # (pack, MMA, sum of parts, twice) and its FP64 products
+    sc = S.ellipsoids_scene(2, 1500, seed=21)
+    plan = F.Plan(sc.y, sc.rho, sc.lam, sc.max_super)
+    s = F.Solver(plan, x=_t(sc.x), nx=_t(sc.nx), y=_t(sc.y), coef=sc.coef, precision=F.MBC_F64).set_fp64_matvec("int8")
+    before = s.launches()
+    s.prepare()
+    assert s.launches() - before == 2 + 2 * 3 + 2
