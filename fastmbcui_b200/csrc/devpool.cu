@@ -174,6 +174,20 @@ mbc_status DevMem::reserve(size_t b)
   return MBC_OK;
 }
 
+mbc_status DevMem::reserve_spare(size_t b)
+{
+  constexpr size_t kSmall = (size_t)64 << 20;  // not asked about
+  if ((b > bytes || !ptr) && b > kSmall) {
+    size_t free_b = 0, total_b = 0;
+    MBC_CK(device_free_bytes(&free_b, &total_b));
+    if (free_b < b + std::max((size_t)4 << 30, total_b / 10)) {
+      release();
+      return fail(MBC_NO_MEMORY, "no spare device memory");
+    }
+  }
+  return reserve(b);
+}
+
 cudaError_t device_free_bytes(size_t *free_b, size_t *total_b)
 {
   const cudaError_t e = cudaMemGetInfo(free_b, total_b);

@@ -51,6 +51,10 @@ struct DevMem {
   DevMem &operator=(const DevMem &) = delete;
   ~DevMem() { release(); }
   mbc_status reserve(size_t b);
+  // ... for memory that only makes a call faster (the parts of split
+  // reductions): refused where it would take the room that the call's other
+  // buffers may need, 4 GiB or a tenth of the device
+  mbc_status reserve_spare(size_t b);
   void release();
 
  private:

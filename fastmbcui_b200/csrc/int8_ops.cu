@@ -280,14 +280,14 @@ mbc_status mbc::Solver::ensure_oz(cudaStream_t st, int R)
     MBC_TRY(m_oz_b.reserve(oz::bimg_bytes(K, std::max(R, 1))));
     MBC_TRY(m_oz_bexp.reserve(sizeof(int32_t) * oz::bexp_count(K, std::max(R, 1))));
     // the check takes the way of the products that follow: parts and their sum
-    if (!oz_slab) m_oz_parts.reserve(oz_parts_bytes(*this, 1));
+    if (!oz_slab) m_oz_parts.reserve_spare(oz_parts_bytes(*this, 1));
     MBC_TRY(oz_selfcheck(st));
   }
   const int K = std::max(n, nf);
   MBC_TRY(m_oz_b.reserve(oz::bimg_bytes(K, R)));
   MBC_TRY(m_oz_bexp.reserve(sizeof(int32_t) * oz::bexp_count(K, R)));
   if (!oz_slab && R > oz_parts_R) {  // sized before any capture; without it products run unsplit
-    m_oz_parts.reserve(oz_parts_bytes(*this, R));
+    m_oz_parts.reserve_spare(oz_parts_bytes(*this, R));
     oz_parts_R = R;
   }
   return MBC_OK;

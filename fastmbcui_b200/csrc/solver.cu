@@ -161,7 +161,7 @@ static void tc_reserve(const Solver &S, int R)
 {
   if (!use_tc(S, R)) return;
   const size_t b = std::max((size_t)tc_parts(S.nf, S.n, R) * S.nf, (size_t)tc_parts(S.n, S.nf, R) * S.n) * R * 4;
-  S.m_tc_parts.reserve(b);  // without it the products run unsplit
+  S.m_tc_parts.reserve_spare(b);  // without it the products run unsplit
 }
 
 template <int DIR>
@@ -194,7 +194,7 @@ static int tc_launch(const Solver &S, int R, const float *vin, float *out, const
   const int smem = tc::smem_bytes(a.np, DIR);  // allowed by use_tc
   const unsigned grid = cdiv(M, tc::kM);
   int parts = tc_parts(M, K, R);
-  if (parts > 1 && S.m_tc_parts.reserve((size_t)parts * M * R * 4) != MBC_OK) parts = 1;
+  if (parts > 1 && S.m_tc_parts.reserve_spare((size_t)parts * M * R * 4) != MBC_OK) parts = 1;
   a.parts = (float *)S.m_tc_parts.ptr;
   tc::pk_tc_kernel<DIR><<<dim3(grid, parts), tc::kThreads, smem, st>>>(a);
   if (parts == 1) return (int)grid;
@@ -394,7 +394,7 @@ static mbc_status launch_grams(Solver &S, const std::vector<int32_t> &ids, T *th
   np = std::min<int64_t>(np, std::max(1, S.nf / 512));
   np = std::min<int64_t>(np, ((int64_t)512 << 20) / std::max<int64_t>(1, len * (int64_t)sizeof(T)));
   np = std::max<int64_t>(1, std::min<int64_t>(np, gram::kMaxParts));
-  if (np > 1 && S.gram_part.reserve((size_t)np * len * sizeof(T)) != MBC_OK) np = 1;
+  if (np > 1 && S.gram_part.reserve_spare((size_t)np * len * sizeof(T)) != MBC_OK) np = 1;
   T *dst = theta;
   g.off = S.d_th_ptr();
   if (np > 1) {

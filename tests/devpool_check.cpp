@@ -221,6 +221,24 @@ void leave()
   CHECK(g_live.empty());
 }
 
+// memory that a call can do without leaves 4 GiB or a tenth of the device, idle
+// memory counted as free; 64 MB are always given
+void spare()
+{
+  mbc::PoolUser user;
+  {
+    DevMem a;
+    CHECK(a.reserve(2 * kGiB) == MBC_OK);
+  }
+  g_other[0] = 54 * kGiB;  // 10 of 64 GiB free, 2 of them idle
+  DevMem x;
+  CHECK(x.reserve_spare(3 * kGiB) == MBC_OK);
+  CHECK(x.reserve_spare(3 * kGiB) == MBC_OK);  // has it already
+  CHECK(x.reserve_spare(5 * kGiB) == MBC_NO_MEMORY && !x.ptr && !x.bytes);
+  g_other[0] = 59 * kGiB;
+  CHECK(x.reserve_spare(kGiB) == MBC_NO_MEMORY && x.reserve_spare(64 * MiB) == MBC_OK);
+}
+
 // with less than a quarter of the device free nothing idle outlives a solver
 void room()
 {
@@ -285,7 +303,7 @@ int main(int argc, char **argv)
 {
   const std::map<std::string, void (*)()> checks = {
       {"reuse", reuse}, {"bound", bound}, {"trim", trim}, {"trim_unpooled", trim_unpooled}, {"leave", leave},
-      {"room", room}, {"waits", waits}, {"host_memory", host_memory}};
+      {"room", room}, {"spare", spare}, {"waits", waits}, {"host_memory", host_memory}};
   auto it = checks.find(argc > 1 ? argv[1] : "");
   if (it == checks.end()) return 2;
   it->second();

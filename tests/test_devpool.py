@@ -26,7 +26,7 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("check", ["reuse", "bound", "trim", "trim_unpooled", "leave", "room", "waits",
+@pytest.mark.parametrize("check", ["reuse", "bound", "trim", "trim_unpooled", "leave", "room", "spare", "waits",
                                    "host_memory"])
 def test_pool(exe, check):
     r = subprocess.run([exe, check], capture_output=True, text=True, timeout=60)
