@@ -75,7 +75,6 @@ int product(const Solver &S, int R, const double *in, double *out, double coef, 
   a.in = in;
   a.out = out;
   a.R = R;
-  a.groups = c.groups;
   a.coef = coef;
   a.pdot = pdot;
   a.part = part;

@@ -31,9 +31,9 @@
 //     order.
 // Positions past the end carry the last point and zero vector entries: their
 // kernel values are finite wherever that point's own are.
-// Measured (B200, K then K^T): 20000 x 20000, 60 columns 4.76 ms, against
+// Measured (B200, K then K^T): 20000 x 20000, 60 columns 4.90 ms, against
 // 10.92 ms for one thread per output with FP64 FMAs and one evaluation per 32
-// columns; the FP64 pipe's floor is 3.3 ms.
+// columns; the FP64 pipe's floor is 3.5 ms.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -58,7 +58,7 @@ struct Args {
   int nf, n;
   const double *in;       // K x R vector block (row stride R)
   double *out;            // M x R
-  int R, groups;
+  int R;
   double coef;
   const double *pdot;     // curvature partials: p, M x R, or NULL
   double *part;           // per slice of outputs: part[(blockIdx.x * cluster size + rank) * R + r]

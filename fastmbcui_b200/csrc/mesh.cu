@@ -76,12 +76,13 @@ __global__ void __launch_bounds__(128) solid_angle_kernel(int n_vert, const floa
 //   * for |num| <= (den - 0.01) / 4 (all but the few sources next to a face or
 //     its edges) takes atan(num / den) from its Maclaurin series, 4 terms below
 //     0.02 and 10 up to 0.25 (errors 3e-15 and 5e-14 of the value); the other
-//     entries take the formula with square roots and atan2.  So do those
-//     where the form above cancels: den by its absolute error of ~3e-13 (y) and
-//     ~3e-16 times the ratio of the longest to the shortest of l1, l2, l3, R1 . n
-//     by that ratio too.  With den at least 0.01 and the ratio at most 256 an
-//     entry keeps 1e-10, a thousandth of the FP32 rounding.  And so do distances outside 1e-17 .. 1e17, whose squares
-//     leave FP32's range, and faces without a vertex (NaN);
+//     entries take the formula with square roots and atan2.  So do those where
+//     the form above cancels: den has an absolute error of ~3e-13 (from y, up to
+//     4e-14 each) and ~3e-16 times the ratio of the longest to the shortest of
+//     l1, l2, l3, and R1 . n loses that ratio too.  With den at least 0.01 and
+//     the ratio at most 256 an entry keeps 1e-10, a thousandth of the FP32
+//     rounding.  Distances outside 1e-17 .. 1e17, whose squares leave FP32's
+//     range, and faces without a vertex (NaN) take the formula as well.
 // About 40 FP64 instructions an entry instead of 190; the error is the FP32
 // rounding of the stored value, as before.  Measured (B200, 30720 x 15372):
 // 4.90 -> 2.49 ms; the FP64 pipe is 40 to 45 % busy, the rest waits for the chains of

@@ -719,7 +719,10 @@ static bool reduce_in_place(int nblk, int R) { return (int64_t)cdiv(nblk, 32) * 
 // The two halves of the preconditioner, z = L (L^T r); with `part` the second
 // forms the partials of r . z and, for mode RED_BETA, their reduction.
 // Warps per row: as many as keep ~16 warps per SM busy in small scenes.  The
-// grid is one wave of resident blocks: six of 256 threads at 40 registers.
+// grid is one wave of resident blocks: six of 256 threads at 40 registers.  Six
+// or eight take the same time (24000-point step 99.2 ms with either); what the
+// choice moves is the order of the sums, and with it, by up to a factor of two,
+// the iterations of FP64 columns that run into their rounding level.
 struct PrecondShape {
   dim3 grid;
   int cx, wpr;
@@ -1081,9 +1084,10 @@ __global__ void block_fail_kernel(int a, const int32_t *__restrict__ act, PcgSca
 // columns the block PCG keeps while any column iterates.  Narrow INT8
 // matvecs are bound by the digit-plane stream, so a wider tail block costs
 // little: at N = 64000 one launch takes 3.4 ms at 16 columns and 4.1 ms at
-// 48.  Measured on the 32-ellipsoid trajectory (8 poses, B200): 48 gives 4.6 %
-// fewer column-iterations and 2.5 % shorter steps than 16; 64 and 96 lower
-// the iterations further but lengthen the steps.
+// 48.  Measured on the 32-ellipsoid trajectory (8 poses, B200, with every INT8
+// product in one part): 48 gives 4.6 % fewer column-iterations and 2.5 %
+// shorter steps than 16; 64 and 96 lower the iterations further but lengthen
+// the steps.
 constexpr int kBlockKeep = 48;
 
 template <typename LT>
