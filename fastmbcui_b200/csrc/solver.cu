@@ -1806,10 +1806,12 @@ mbc_status Solver::solve(int R, const void *rhs, int32_t rhs_dt, void *X, int32_
     // one cold-started PCG per column, in order (mfs_torch_ops.cu:166-171)
     const size_t rows = adjoint ? (size_t)n : (size_t)nf;
     const size_t ein = rhs_dt == MBC_F64 ? 8 : 4, eout = x_dt == MBC_F64 ? 8 : 4;
-    MBC_TRY(colbuf.reserve(rows * ein + (size_t)n * eout * 2));
+    // aligned for FP64 values behind an odd number of FP32 ones
+    const size_t in_b = (rows * ein + 255) & ~(size_t)255, out_b = ((size_t)n * eout + 255) & ~(size_t)255;
+    MBC_TRY(colbuf.reserve(in_b + 2 * out_b));
     char *cin = (char *)colbuf.ptr;
-    char *cx0 = cin + rows * ein;
-    char *cout = cx0 + (size_t)n * eout;
+    char *cx0 = cin + in_b;
+    char *cout = cx0 + out_b;
     mbc_solve_stats agg{};
     agg.true_relres_max = -1;
     int worst = 0;
