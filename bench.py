@@ -277,8 +277,8 @@ def run_trajectory(args):
 
     # accuracy of the timed path: every column's FP64 true residual
     # |K^T (f - K x)| / |K^T f| of the last timed step, recomputed after the
-    # timing with the FP64 CUDA-core kernels (the ones the parity tests pin to
-    # the oracle)
+    # timing with the FP64 kernels (the ones the parity tests pin to the
+    # oracle)
     k_last = args.warmup + len(times) - 1
     s64 = F.Solver(plans[k_last], x=coords[k_last][0], nx=coords[k_last][1], y=coords[k_last][2],
                    coef=base.coef, precision=F.MBC_F64)
@@ -286,8 +286,8 @@ def run_trajectory(args):
     nb = torch.linalg.norm(s64.apply_KT(f64), dim=0)
     rel = torch.linalg.norm(s64.apply_KT(f64 - s64.apply_K(X)), dim=0) / torch.clamp(nb, min=1e-300)
     verify = {"true_relres_max": _max_over_ranks(dist, float(rel.max())), "tol": 1e-8, "columns": R,
-              "step": k_last, "how": "FP64 CUDA-core K and K^T after the timed steps, on the last timed "
-                                     "step's strengths"}
+              "step": k_last, "how": "FP64 K and K^T after the timed steps, on the last timed step's "
+                                     "strengths"}
     del s64, f64
 
     # end to end through the public API, continuing the trajectory: host
@@ -348,7 +348,7 @@ def run_trajectory(args):
         "clocks": clk.summary(),
     }
     # the plain FP64 method (the reference's algorithm in FP64: one cold PCG
-    # per column, FP64 factor, FP64 CUDA-core matvec) on the trajectory's first
+    # per column, FP64 factor, FP64 matvec) on the trajectory's first
     # pose, the pose of the CPU oracle's iteration fixture
     if _left(args) > args.reserve_s * 0.5:
         out["plain_fp64"] = _plain_leg(args, F, plans[0] if args.plan_every == 1 else None, scenes[0], t, R)
@@ -382,7 +382,7 @@ WARM = {"learned": "quadratic extrapolation + MLP correction (3x256, BF16 weight
 
 def _plain_leg(args, F, plan, sc, t, R):
     """The plain FP64 method on one pose: FP64 factor, then one cold FP64 PCG
-    per column (FP64 CUDA-core matvec), the oracle fixture's columns first,
+    per column (FP64 matvec), the oracle fixture's columns first,
     for at most --plain-s seconds (at least two columns); the mean time per
     column is extrapolated to all R."""
     import torch
@@ -430,10 +430,10 @@ def _plain_leg(args, F, plan, sc, t, R):
 def _ablation(args, F, TS, base, sc, t, plain, ts_main):
     """Where the speed-up comes from, on one fresh pose of the trajectory
     (the pose after the ones already solved; solves/s):
-      plain     per-RHS cold FP64 PCG, FP64 CUDA-core matvec, FP64 factor
+      plain     per-RHS cold FP64 PCG, FP64 matvec, FP64 factor
                 (the plain leg, measured on the first pose);
       batched   all R columns in one cold batched FP64 PCG on the FP64
-                CUDA-core matvec: 16 iterations timed, scaled to the
+                matvec: 16 iterations timed, scaled to the
                 iterations of the same batched solve on the INT8 matvec (the
                 same per-column recurrences);
       int8      that batched cold solve on the INT8 tensor-core matvec, timed;
@@ -772,7 +772,7 @@ def run_ours(args):
     block PCG, FP64-accurate INT8 matvec; for the large scene the digit
     planes do not fit and are rebuilt slab by slab for every matvec).  The
     host plan is its own column; the FP64 true residual of the result is
-    checked with the FP64 CUDA-core kernels."""
+    checked with the FP64 kernels."""
     import torch
 
     import fastmbcui_b200 as F
@@ -825,7 +825,7 @@ def run_ours(args):
                 break
     ms_step = _max_over_ranks(dist, float(np.mean(times)))
     value = world * 1000.0 / ms_step
-    # FP64 true residual of the result (FP64 CUDA-core kernels)
+    # FP64 true residual of the result (FP64 kernels)
     s64 = F.Solver(plan, x=x, nx=nx, y=y, coef=sc.coef, precision=F.MBC_F64)
     F64 = Fd.double()
     b = s64.apply_KT(F64)
@@ -1138,7 +1138,7 @@ def main():
                     help="time the adjoint solve, the op bodies' cache, the added mass and the mesh assembly "
                          "(one JSON line each)")
     ap.add_argument("--fp64-matvec", default="int8", choices=["simt", "int8"],
-                    help="FP64 matvec: CUDA-core FP64 kernels or exact INT8 digit slicing on the tensor cores")
+                    help="FP64 matvec: FP64 kernels or exact INT8 digit slicing on the tensor cores")
     args = ap.parse_args()
     if args.rows_probe:
         run_rows(args)
