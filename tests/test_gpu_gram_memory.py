@@ -3,12 +3,15 @@ Theta for the parts of its rows, not of the whole scene's: the device memory tha
 factor() takes is that of its results (Theta in FP32 and FP64, L twice), plus
 64 MB of lists, workspaces and granularity.  In a process of its own, where no
 other solver is alive."""
+import os
 import subprocess
 import sys
 
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 PROG = """
 import numpy as np, torch
@@ -36,5 +39,5 @@ print("ok")
 
 
 def test_retry_of_few_sets_takes_little_memory():
-    r = subprocess.run([sys.executable, "-c", PROG], capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", PROG], capture_output=True, text=True, timeout=300, cwd=ROOT)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), (r.stdout, r.stderr[-2000:])

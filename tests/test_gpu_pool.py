@@ -5,12 +5,15 @@ the device.  In a process of its own, where no other solver is alive.
 The larger scene's solver has over 60 MB; the device's free memory after a small
 call may fall short of that before the larger one by 32 MB (the kernels' code, the
 small solver, allocation granularity)."""
+import os
 import subprocess
 import sys
 
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 PROG = """
 import numpy as np, torch
@@ -39,5 +42,5 @@ print("ok")
 
 
 def test_operator_calls_keep_no_idle_memory():
-    r = subprocess.run([sys.executable, "-c", PROG], capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", PROG], capture_output=True, text=True, timeout=300, cwd=ROOT)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), (r.stdout, r.stderr[-2000:])
